@@ -8,10 +8,6 @@
 // fftw_execute_dft(ifft_plan) / cipow step / w=0 transfer / fft_plan sequence of
 // src/reference/grid.c:467-499 with the per-floor row transforms done by the
 // row kernel beforehand.
-//
-// FP64 (image formation, any n <= 4096): radix-2 Stockham rows in shared
-// memory for powers of two, Bluestein's algorithm (k_bluestein.cu) for other
-// lengths, plus tiled transposes; not on the timed path.
 #include <cmath>
 #include <vector>
 
@@ -753,102 +749,6 @@ void launch_tower_finish(cudaStream_t s, int group_cap, const int *tower_group_f
                                        subimg, tw)
     RG_DISPATCH_N1(subgrid, CALL)
 #undef CALL
-}
-
-// ---------------------------------------------------------------------------
-// FP64 transforms (image formation)
-// ---------------------------------------------------------------------------
-bool fft64_supported(int n) { return n >= 2 && n <= 4096 && (n & (n - 1)) == 0; }
-
-// One row per CTA: radix-2 Stockham autosort in shared memory (ping-pong),
-// twiddles from an FP64 table exp(-2 pi i k / n), k < n/2.
-__global__ void fft64_rows_kernel(double2 *__restrict__ data, int n, int sign,
-                                  const double2 *__restrict__ tw)
-{
-    extern __shared__ double2 sm64[];
-    double2 *a = sm64, *b = sm64 + n;
-    double2 *row = data + (int64_t)blockIdx.x * n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = row[i];
-    __syncthreads();
-    const int half = n / 2;
-    // Stockham radix-2 autosort: sub-transforms of length Ns double each pass
-    for (int Ns = 1; Ns < n; Ns <<= 1) {
-        for (int t = threadIdx.x; t < half; t += blockDim.x) {
-            const int k = t % Ns;
-            double2 w = tw[k * (n / (2 * Ns))];
-            if (sign > 0) w.y = -w.y;
-            const double2 x = a[t];
-            const double2 y = a[t + half];
-            const double2 ty = make_double2(w.x * y.x - w.y * y.y, w.x * y.y + w.y * y.x);
-            const int d = (t / Ns) * Ns * 2 + k;
-            b[d] = make_double2(x.x + ty.x, x.y + ty.y);
-            b[d + Ns] = make_double2(x.x - ty.x, x.y - ty.y);
-        }
-        __syncthreads();
-        double2 *t2 = a; a = b; b = t2;
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) row[i] = a[i];
-}
-
-__global__ void transpose64_kernel(const double2 *__restrict__ in, double2 *__restrict__ out,
-                                   int ny, int nx)
-{
-    __shared__ double2 tile[32][33];
-    const int64_t off = (int64_t)blockIdx.z * ny * nx;
-    int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 32 + threadIdx.y;
-    for (int k = 0; k < 32; k += 8)
-        if (x < nx && y + k < ny) tile[threadIdx.y + k][threadIdx.x] = in[off + (int64_t)(y + k) * nx + x];
-    __syncthreads();
-    x = blockIdx.y * 32 + threadIdx.x;
-    y = blockIdx.x * 32 + threadIdx.y;
-    for (int k = 0; k < 32; k += 8)
-        if (x < ny && y + k < nx) out[off + (int64_t)(y + k) * ny + x] = tile[threadIdx.x][threadIdx.y + k];
-}
-
-static double2 *twiddles64(cudaStream_t s, int n)
-{
-    // one table per size per process (small; kept for reuse)
-    static std::map<int, double2 *> cache;
-    auto it = cache.find(n);
-    if (it != cache.end()) return it->second;
-    std::vector<double2> h(n / 2 > 0 ? n / 2 : 1);
-    for (int k = 0; k < n / 2; k++) {
-        double a = -2.0 * M_PI * (double)k / (double)n;
-        h[k] = make_double2(std::cos(a), std::sin(a));
-    }
-    double2 *d = nullptr;
-    cudaMalloc(&d, sizeof(double2) * h.size());
-    cudaMemcpyAsync(d, h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice, s);
-    cudaStreamSynchronize(s);
-    cache[n] = d;
-    return d;
-}
-
-const double2 *fft64_twiddles(cudaStream_t s, int n) { return twiddles64(s, n); }
-
-static void rows64(cudaStream_t s, double2 *data, int64_t rows, int n, int sign)
-{
-    const size_t sm = sizeof(double2) * 2 * n;
-    cudaFuncSetAttribute(fft64_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    const int threads = n / 2 < 512 ? (n / 2 > 32 ? n / 2 : 32) : 512;
-    fft64_rows_kernel<<<(unsigned)rows, threads, sm, s>>>(data, n, sign, twiddles64(s, n));
-}
-
-void launch_fft64_pow2_rows(cudaStream_t s, double2 *data, int64_t rows, int n, int sign)
-{
-    rows64(s, data, rows, n, sign);
-}
-
-void launch_fft64_2d(cudaStream_t s, double2 *data, double2 *tmp, int batch, int ny, int nx, int sign,
-                     double2 *work)
-{
-    launch_fft64_any_rows(s, data, (int64_t)batch * ny, nx, sign, work);
-    dim3 blk(32, 8);
-    dim3 g1((nx + 31) / 32, (ny + 31) / 32, batch);
-    transpose64_kernel<<<g1, blk, 0, s>>>(data, tmp, ny, nx);
-    launch_fft64_any_rows(s, tmp, (int64_t)batch * nx, ny, sign, work);
-    dim3 g2((ny + 31) / 32, (nx + 31) / 32, batch);
-    transpose64_kernel<<<g2, blk, 0, s>>>(tmp, data, nx, ny);
 }
 
 }  // namespace rg

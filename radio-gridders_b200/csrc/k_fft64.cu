@@ -1,0 +1,214 @@
+// Plans and launches of the FP64 transforms (k_fft64.cuh): in-place 2-D
+// transforms and the dirty image's two passes.
+//
+// Both passes are bound by memory and by the latency of one CTA's
+// load - transform - store sequence, with the FP64 pipe behind them
+// (5 n^2 log2 n^2 operations: 0.7 GFLOP at n = 2500). One image of a 2500 x 2500
+// grid, with the caller's copy of the grid: 483 us, against 4522 us as
+// hermitian, shift, radix-2 Bluestein rows, transpose, rows, transpose, shift
+// and real part, each a pass of its own.
+#include <algorithm>
+#include <string>
+
+#include "k_fft64.cuh"
+
+namespace rg {
+
+bool fft64_any_supported(int n) { return n >= 2 && n <= 4096; }
+
+// Splits L into stages; false if it has a prime factor above 7. Powers of two
+// as 16s, the rest as one 8, 4 or 2, or as 8s where that leaves no 2; odd radices
+// first: their first stage stores with an odd stride, free of bank conflicts.
+static bool fft64_stages(int L, Fft64Plan *p)
+{
+    int n = L, lg = 0;
+    p->nst = 0;
+    for (int r : {7, 5, 3})
+        while (n % r == 0) {
+            n /= r;
+            p->radix[p->nst++] = r;
+        }
+    while (n % 2 == 0) {
+        n /= 2;
+        lg++;
+    }
+    if (n != 1) return false;
+    while (lg > 0) {
+        const int e = lg == 5 || lg == 6 || lg == 9 ? 3 : std::min(lg, 4);
+        p->radix[p->nst++] = 1 << e;
+        lg -= e;
+    }
+    p->L = L;
+    int64_t ns = 1;
+    for (int k = 0; k < p->nst; k++) {
+        p->magic[k] = ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0u;
+        ns *= p->radix[k];
+    }
+    return true;
+}
+
+// tw[k] = exp(-2 pi i k / L)
+__global__ void fft64_twiddle_kernel(double2 *__restrict__ tw, int L)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= L) return;
+    double s, c;
+    sincospi(-2.0 * (double)k / (double)L, &s, &c);
+    tw[k] = make_double2(c, s);
+}
+
+// chirp[m] = exp(-pi i m^2 / n), the phase reduced exactly (m^2 mod 2n in
+// integers), and the filter before its transform: conj(chirp) wrapped to
+// length L (it is even in m), zero between.
+__global__ void fft64_chirp_kernel(double2 *__restrict__ chirp, double2 *__restrict__ wrapped, int n, int L)
+{
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= L) return;
+    const int d = m < n ? m : L - m;
+    double2 v = make_double2(0.0, 0.0);
+    if (d < n) {
+        const long long q = ((long long)d * d) % (2LL * n);
+        double s, c;
+        sincospi(-(double)q / (double)n, &s, &c);
+        v = make_double2(c, -s);
+        if (m < n) chirp[m] = make_double2(c, s);
+    }
+    wrapped[m] = v;
+}
+
+struct LdRows {
+    const double2 *d;
+    int64_t ld;
+    __device__ double2 operator()(int, int line, int n) const { return d[line * ld + n]; }
+};
+struct StRows {
+    double2 *d;
+    int64_t ld;
+    __device__ void operator()(int, int line, int n, double2 v) const { d[line * ld + n] = v; }
+};
+struct LdCols {
+    const double2 *d;
+    int64_t ld, array;
+    __device__ double2 operator()(int arr, int line, int n) const { return d[arr * array + n * ld + line]; }
+};
+struct StCols {
+    double2 *d;
+    int64_t ld, array;
+    __device__ void operator()(int arr, int line, int n, double2 v) const { d[arr * array + n * ld + line] = v; }
+};
+
+rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
+{
+    auto it = ctx->fft64_plans.find(n);
+    if (it != ctx->fft64_plans.end()) {
+        *out = it->second;
+        return RG_OK;
+    }
+    Fft64Plan p;
+    p.n = n;
+    bool direct = fft64_stages(n, &p);
+    if (!direct) {
+        // the cheapest convolution length: points times passes over them, of
+        // those whose stages fit one CTA's threads
+        Fft64Plan best;
+        int64_t cost = INT64_MAX;
+        for (int L = 2 * n - 1; L <= 8192; L++) {
+            Fft64Plan c;
+            if (!fft64_stages(L, &c) || fft64_threads(c, 0) > 512) continue;
+            if ((int64_t)L * (c.nst + 1) < cost) {
+                cost = (int64_t)L * (c.nst + 1);
+                best = c;
+            }
+        }
+        p = best;
+        p.n = n;
+    }
+    p.scale = 1.0 / (double)p.L;
+    // one buffer: twiddles, then for Bluestein the filter and the chirp
+    const size_t elems = (size_t)p.L * (direct ? 1 : 2) + (direct ? 0 : n);
+    void *mem;
+    RG_CHECK(scratch(ctx, ("fft64_" + std::to_string(n)).c_str(), sizeof(double2) * elems, &mem));
+    double2 *tw = (double2 *)mem;
+    p.tw = tw;
+    fft64_twiddle_kernel<<<(p.L + 127) / 128, 128, 0, ctx->stream>>>(tw, p.L);
+    if (!direct) {
+        double2 *filter = tw + p.L, *chirp = filter + p.L;
+        fft64_chirp_kernel<<<(p.L + 127) / 128, 128, 0, ctx->stream>>>(chirp, filter, n, p.L);
+        Fft64Plan q = p;  // the L-point transform of the filter
+        q.n = p.L;
+        launch_fft64_lines<false>(ctx->stream, q, 1, 1, -1, LdRows{filter, p.L}, StRows{filter, p.L});
+        p.filter = filter;
+        p.chirp = chirp;
+    }
+    RG_CUDA(cudaGetLastError());
+    ctx->fft64_plans[n] = p;
+    *out = p;
+    return RG_OK;
+}
+
+void launch_fft64_2d(cudaStream_t s, double2 *data, int batch, const Fft64Plan &py, const Fft64Plan &px, int sign)
+{
+    const int ny = py.n, nx = px.n;
+    launch_fft64_lines<false>(s, px, 1, batch * ny, sign, LdRows{data, nx}, StRows{data, nx});
+    launch_fft64_lines<true>(s, py, batch, nx, sign, LdCols{data, nx, (int64_t)ny * nx},
+                             StCols{data, nx, (int64_t)ny * nx});
+}
+
+// Rows of the dirty image: line 2p is grid row p and line 2p + 1 its mirror
+// N - p (pair 0: rows 0 and N/2), so the two rows of a hermitian pair are read
+// at the same time and the second read of each comes from L2. The point read
+// is the hermitian sum of src/reference/grid.c:639-662 (linear index i >= N + 1
+// pairs with N^2 + N - i; row 0 and element (1, 0) are left as they are) at
+// the shifted column (grid.c:665-680); the row goes to its shifted place.
+struct LdImageRow {
+    const double2 *g;
+    int N;
+    __device__ int row(int line) const
+    {
+        const int p = line >> 1;
+        return line & 1 ? (p == 0 ? N / 2 : N - p) : p;
+    }
+    __device__ double2 operator()(int, int line, int n) const
+    {
+        const int y = row(line), x = n < N / 2 ? n + N / 2 : n - N / 2;
+        const int64_t i = (int64_t)y * N + x;
+        const double2 a = g[i];
+        if (i < N + 1) return a;
+        const double2 b = g[(int64_t)N * N + N - i];
+        return make_double2(a.x + b.x, a.y - b.y);
+    }
+};
+struct StImageRow {
+    double2 *tmp;
+    int N;
+    __device__ void operator()(int, int line, int n, double2 v) const
+    {
+        const int p = line >> 1;
+        const int y = line & 1 ? (p == 0 ? N / 2 : N - p) : p;
+        tmp[(int64_t)(y < N / 2 ? y + N / 2 : y - N / 2) * N + n] = v;
+    }
+};
+// Columns: the transformed grid and the image at their shifted places.
+struct StImageCol {
+    double2 *g;
+    double *img;
+    const double *taper;
+    int N;
+    __device__ void operator()(int, int line, int n, double2 v) const
+    {
+        const int y = n < N / 2 ? n + N / 2 : n - N / 2, x = line < N / 2 ? line + N / 2 : line - N / 2;
+        const int64_t i = (int64_t)y * N + x;
+        g[i] = v;
+        img[i] = taper ? v.x / (__ldg(taper + y) * __ldg(taper + x)) : v.x;
+    }
+};
+
+void launch_image_from_grid(cudaStream_t s, double2 *grid, double2 *tmp, double *image, const double *taper,
+                            const Fft64Plan &p)
+{
+    const int N = p.n;
+    launch_fft64_lines<false>(s, p, 1, N, -1, LdImageRow{grid, N}, StImageRow{tmp, N});
+    launch_fft64_lines<true>(s, p, 1, N, -1, LdCols{tmp, N, 0}, StImageCol{grid, image, taper, N});
+}
+
+}  // namespace rg

@@ -1,5 +1,5 @@
 // Element-wise and image-formation kernels: kernel-table conversion, uniform
-// weighting, make_hermitian, fft_shift, real part / grid correction, and the
+// weighting, make_hermitian, fft_shift, and the
 // FP32 -> FP64 grid accumulation of the W-projection path.
 #include "rg_internal.h"
 
@@ -116,23 +116,6 @@ __global__ void fft_shift_kernel(double2 *__restrict__ g, int n)
 void launch_fft_shift(cudaStream_t s, double2 *grid, int n)
 {
     fft_shift_kernel<<<blocks_for((int64_t)n * (n / 2)), 256, 0, s>>>(grid, n);
-}
-
-__global__ void real_part_kernel(const double2 *__restrict__ g, double *__restrict__ img, int n,
-                                 const double *__restrict__ taper)
-{
-    const int64_t total = (int64_t)n * n;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        double v = g[k].x;
-        if (taper) v /= taper[k / n] * taper[k % n];
-        img[k] = v;
-    }
-}
-
-void launch_real_part(cudaStream_t s, const double2 *grid, double *img, int n, const double *taper)
-{
-    real_part_kernel<<<blocks_for((int64_t)n * n), 256, 0, s>>>(grid, img, n, taper);
 }
 
 // nearest cell, src/reference/grid.c:27-35 (index checked here; the

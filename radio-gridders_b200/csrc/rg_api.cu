@@ -1317,14 +1317,9 @@ rg_status rg_image_from_grid(rg_context *ctx, double *uvgrid, int grid_size, dou
     if (taper_1d) RG_CHECK(stage_in(ctx, taper_1d, sizeof(double) * N, "img_taper", &taper));
     OutView img;
     RG_CHECK(out_view(ctx, image_out, sizeof(double) * (size_t)cells, "img_out", false, &img));
-    launch_make_hermitian(ctx->stream, (double2 *)g.dev, N);
-    launch_fft_shift(ctx->stream, (double2 *)g.dev, N);
-    void *work = nullptr;
-    if (fft64_any_work_elems(N) > 0)
-        RG_CHECK(scratch(ctx, "fft64_work", sizeof(double2) * (size_t)fft64_any_work_elems(N), &work));
-    launch_fft64_2d(ctx->stream, (double2 *)g.dev, (double2 *)tmp, 1, N, N, -1, (double2 *)work);
-    launch_fft_shift(ctx->stream, (double2 *)g.dev, N);
-    launch_real_part(ctx->stream, (const double2 *)g.dev, (double *)img.dev, N, (const double *)taper);
+    Fft64Plan plan;
+    RG_CHECK(fft64_plan(ctx, N, &plan));
+    launch_image_from_grid(ctx->stream, (double2 *)g.dev, (double2 *)tmp, (double *)img.dev, (const double *)taper, plan);
     RG_CHECK(check_launch("image formation"));
     RG_CHECK(finish_out(ctx, g));
     RG_CHECK(finish_out(ctx, img));
@@ -1354,12 +1349,10 @@ rg_status rg_fft2d(rg_context *ctx, void *data, int batch, int ny, int nx, int s
             return fail(RG_ERR_UNSUPPORTED, "FP64 transforms need sizes in [2, 4096]");
         OutView ov;
         RG_CHECK(out_view(ctx, data, bytes, "fft_data", true, &ov));
-        void *tmp;
-        RG_CHECK(scratch(ctx, "fft_tmp", bytes, &tmp));
-        const int64_t wel = std::max(fft64_any_work_elems(nx), fft64_any_work_elems(ny));
-        void *work = nullptr;
-        if (wel > 0) RG_CHECK(scratch(ctx, "fft64_work", sizeof(double2) * (size_t)wel, &work));
-        launch_fft64_2d(ctx->stream, (double2 *)ov.dev, (double2 *)tmp, batch, ny, nx, sign, (double2 *)work);
+        Fft64Plan px, py;
+        RG_CHECK(fft64_plan(ctx, nx, &px));
+        RG_CHECK(fft64_plan(ctx, ny, &py));
+        launch_fft64_2d(ctx->stream, (double2 *)ov.dev, batch, py, px, sign);
         RG_CHECK(check_launch("fft64"));
         RG_CHECK(finish_out(ctx, ov));
     } else {

@@ -88,6 +88,22 @@ struct TowerPlan {
     const unsigned char *tower_sel = nullptr;  // device: the towers this plan grids (nullptr: all)
 };
 
+namespace rg {
+
+// The tables of one length: L = n where n's prime factors are at most 7, else
+// the convolution length of Bluestein's algorithm (chirp and filter set).
+struct Fft64Plan {
+    int n = 0, L = 0, nst = 0;
+    int radix[12] = {};       // the stages' radices
+    unsigned magic[12] = {};  // ceil(2^32 / Ns): a stage's j / Ns by one high multiply
+    const double2 *tw = nullptr;      // exp(-2 pi i k / L), k < L
+    const double2 *chirp = nullptr;   // exp(-pi i m^2 / n), m < n
+    const double2 *filter = nullptr;  // transform of the wrapped conj(chirp), L points
+    double scale = 1.0;               // 1 / L
+};
+
+}  // namespace rg
+
 struct rg_stage_event {
     std::string name;
     cudaEvent_t start = nullptr, stop = nullptr;
@@ -105,6 +121,7 @@ struct rg_context {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     std::map<std::string, rg::Buffer> scratch;
+    std::map<int, rg::Fft64Plan> fft64_plans;  // by length; their tables lie in scratch
     uint64_t scratch_gen = 0;  // bumped on every scratch (re)allocation: captured graphs go stale
     // batched W-towers calls: copy streams, their events, per-step diagnostics
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
@@ -189,8 +206,6 @@ void launch_convert_table(cudaStream_t s, const double2 *src, float2 *dst, int64
 void launch_convert_table_dup(cudaStream_t s, const double2 *src, float2 *dst, int64_t n, int kk);
 void launch_make_hermitian(cudaStream_t s, double2 *grid, int n);
 void launch_fft_shift(cudaStream_t s, double2 *grid, int n);
-void launch_real_part(cudaStream_t s, const double2 *grid, double *img, int n,
-                      const double *taper);
 void launch_weight_count(cudaStream_t s, const double *u, const double *v, int64_t nvis,
                          int n, double theta, unsigned *count);
 void launch_weight_apply(cudaStream_t s, const double *u, const double *v,
@@ -212,18 +227,17 @@ void launch_fft32_rows(cudaStream_t s, float2 *data, int64_t rows, int n, int si
 // left as they are (live may be NULL: all)
 void launch_fft32_cols(cudaStream_t s, float2 *data, int batch, int n, int sign,
                        const float2 *tw, const int *live = nullptr);
-// FP64 transforms for image formation: power-of-two n <= 4096 directly,
-// any other n <= 4096 by Bluestein's algorithm (k_bluestein.cu), which needs
-// fft64_any_work_elems(n) double2 of work space (0 for powers of two).
-bool fft64_supported(int n);
+// k_fft64.cu — FP64 transforms of any length n <= 4096 (k_fft64.cuh)
 bool fft64_any_supported(int n);
-constexpr int kBluesteinRows = 512;  // rows per Bluestein chunk (work space)
-int64_t fft64_any_work_elems(int n);
-const double2 *fft64_twiddles(cudaStream_t s, int n);  // exp(-2 pi i k / n), k < n/2 (cached)
-void launch_fft64_pow2_rows(cudaStream_t s, double2 *data, int64_t rows, int n, int sign);
-void launch_fft64_any_rows(cudaStream_t s, double2 *data, int64_t rows, int n, int sign, double2 *work);
-void launch_fft64_2d(cudaStream_t s, double2 *data, double2 *tmp, int batch, int ny, int nx,
-                     int sign, double2 *work = nullptr);
+// The context's plan for length n (its tables are made on the first call).
+rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out);
+// In-place 2-D transforms of `batch` ny x nx arrays.
+void launch_fft64_2d(cudaStream_t s, double2 *data, int batch, const Fft64Plan &py, const Fft64Plan &px, int sign);
+// The dirty image of an n x n grid (n even): hermitian sum, shift, transform
+// (sign -1), shift; the result goes to grid and its real part, over
+// taper[y] taper[x] if given, to image. tmp: n x n.
+void launch_image_from_grid(cudaStream_t s, double2 *grid, double2 *tmp, double *image, const double *taper,
+                            const Fft64Plan &p);
 
 // k_prepare.cu
 struct TowerGeom {

@@ -220,14 +220,13 @@ extern "C" rg_status rg_wstack_predict(rg_context *ctx, double theta, double lam
         hval[s] = sky[s].re;
         hpix[s] = make_int2(sky[s].x, sky[s].y);
     }
-    void *stack, *tmp, *sidx, *sval, *spix, *work = nullptr;
+    void *stack, *sidx, *sval, *spix;
     RG_CHECK(scratch(ctx, "wstack_planes", sizeof(double2) * g2 * planes, &stack));
-    RG_CHECK(scratch(ctx, "wstack_tmp", sizeof(double2) * g2 * planes, &tmp));
     RG_CHECK(scratch(ctx, "wstack_sky_idx", sizeof(int64_t) * (nsrc + 1), &sidx));
     RG_CHECK(scratch(ctx, "wstack_sky_val", sizeof(double) * (nsrc + 1), &sval));
     RG_CHECK(scratch(ctx, "wstack_sky_pix", sizeof(int2) * (nsrc + 1), &spix));
-    if (fft64_any_work_elems(G) > 0)
-        RG_CHECK(scratch(ctx, "fft64_work", sizeof(double2) * (size_t)fft64_any_work_elems(G), &work));
+    Fft64Plan plan;
+    RG_CHECK(fft64_plan(ctx, G, &plan));
     const void *tuv, *tw;
     RG_CHECK(stage_in(ctx, conv_uv->data, sizeof(double) * (size_t)suv * conv_uv->oversampling, "wstack_conv_uv", &tuv));
     RG_CHECK(stage_in(ctx, conv_w->data, sizeof(double) * (size_t)sw * conv_w->oversampling, "wstack_conv_w", &tw));
@@ -254,7 +253,7 @@ extern "C" rg_status rg_wstack_predict(rg_context *ctx, double theta, double lam
     }
     end_stage(ctx);
     begin_stage(ctx, "wstack_fft");
-    launch_fft64_2d(ctx->stream, (double2 *)stack, (double2 *)tmp, planes, G, G, -1, (double2 *)work);
+    launch_fft64_2d(ctx->stream, (double2 *)stack, planes, plan, plan, -1);
     for (int p = 0; p < planes; p++) launch_fft_shift(ctx->stream, (double2 *)stack + g2 * p, G);
     ctx->launches += 4 + planes;
     end_stage(ctx);

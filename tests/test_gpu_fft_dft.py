@@ -48,6 +48,37 @@ def test_fft64_any_length_vs_numpy(ctx, ny, nx, sign):
     assert rel_rms(y, ref) < 1e-12
 
 
+@pytest.mark.parametrize("batch,ny,nx", [(1, 2, 3), (5, 7, 5), (2, 11, 13), (3, 49, 17), (2, 128, 243), (1, 625, 121),
+                                         (2, 2187, 66), (1, 70, 2401), (1, 3, 4093), (1, 4093, 5), (1, 4050, 9),
+                                         (1, 10, 4096), (1, 4095, 2), (300, 4, 16), (1, 1030, 1000)])
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_fft64_stage_mixes_vs_numpy(ctx, batch, ny, nx, sign):
+    """Every radix alone and mixed, one stage and many, prime lengths up to the
+    longest convolution, ragged column groups and batches. FP64 rounding grows
+    with the stages (< 1e-15 each here); the tolerance is the one above."""
+    rng = np.random.default_rng(ny * 4099 + nx)
+    x = rng.normal(size=(batch, ny, nx)) + 1j * rng.normal(size=(batch, ny, nx))
+    y = x.copy()
+    ctx.fft2d(y, sign)
+    ref = np.fft.fft2(x) if sign < 0 else np.fft.ifft2(x) * (nx * ny)
+    assert rel_rms(y, ref) < 1e-12
+
+
+@pytest.mark.parametrize("n", [2, 4, 6, 22, 34, 250, 1024, 1030])
+@pytest.mark.parametrize("tapered", [False, True])
+def test_image_from_grid_vs_oracle(ctx, oracle, n, tapered):
+    """The two-pass image (hermitian sum, shifts and taper on the way) against
+    the oracle's hermitian and shift with numpy's FFT, the transformed grid too."""
+    rng = np.random.default_rng(n)
+    g = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+    taper = rng.uniform(0.5, 1.0, n) if tapered else None
+    full = oracle.fft_shift(np.fft.fft2(oracle.fft_shift(oracle.make_hermitian(g.copy()))))
+    ref = full.real / (taper[:, None] * taper[None, :]) if tapered else full.real
+    out = g.copy()
+    img = ctx.image_from_grid(out, taper_1d=taper)
+    assert rel_rms(out, full) < 1e-12 and rel_rms(img, ref) < 1e-12
+
+
 def test_image_at_a_grid_size_that_is_not_a_power_of_two(rg, ctx, sim, oracle):
     """grid.out's grid size is floor(lambda * theta): theta 0.1, lambda 25000
     gives 2500.  W-projection grid against the oracle, and the dirty image
