@@ -16,6 +16,13 @@ namespace rg {
 
 bool fft64_any_supported(int n) { return n >= 2 && n <= 4096; }
 
+bool fft64_smooth(int n)
+{
+    for (int r : {2, 3, 5, 7})
+        while (n % r == 0) n /= r;
+    return n == 1;
+}
+
 // Splits L into stages; false if it has a prime factor above 7. Powers of two
 // as 16s, the rest as one 8, 4 or 2, or as 8s where that leaves no 2; odd radices
 // first: their first stage stores with an odd stride, free of bank conflicts.
@@ -97,6 +104,18 @@ struct StCols {
     __device__ void operator()(int arr, int line, int n, double2 v) const { d[arr * array + n * ld + line] = v; }
 };
 
+rg_status roots64(rg_context *ctx, int n, const double2 **out)
+{
+    const std::string name = "roots64_" + std::to_string(n);
+    const auto known = ctx->scratch.find(name);
+    const bool fresh = known == ctx->scratch.end() || !known->second.ptr;
+    void *mem;
+    RG_CHECK(scratch(ctx, name.c_str(), sizeof(double2) * (size_t)n, &mem));
+    if (fresh) fft64_twiddle_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>((double2 *)mem, n);
+    *out = (const double2 *)mem;
+    return RG_OK;
+}
+
 rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
 {
     auto it = ctx->fft64_plans.find(n);
@@ -124,15 +143,11 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
         p.n = n;
     }
     p.scale = 1.0 / (double)p.L;
-    // one buffer: twiddles, then for Bluestein the filter and the chirp
-    const size_t elems = (size_t)p.L * (direct ? 1 : 2) + (direct ? 0 : n);
-    void *mem;
-    RG_CHECK(scratch(ctx, ("fft64_" + std::to_string(n)).c_str(), sizeof(double2) * elems, &mem));
-    double2 *tw = (double2 *)mem;
-    p.tw = tw;
-    fft64_twiddle_kernel<<<(p.L + 127) / 128, 128, 0, ctx->stream>>>(tw, p.L);
+    RG_CHECK(roots64(ctx, p.L, &p.tw));
     if (!direct) {
-        double2 *filter = tw + p.L, *chirp = filter + p.L;
+        void *mem;
+        RG_CHECK(scratch(ctx, ("chirp64_" + std::to_string(n)).c_str(), sizeof(double2) * (size_t)(p.L + n), &mem));
+        double2 *filter = (double2 *)mem, *chirp = filter + p.L;
         fft64_chirp_kernel<<<(p.L + 127) / 128, 128, 0, ctx->stream>>>(chirp, filter, n, p.L);
         Fft64Plan q = p;  // the L-point transform of the filter
         q.n = p.L;

@@ -229,6 +229,9 @@ void launch_fft32_cols(cudaStream_t s, float2 *data, int batch, int n, int sign,
                        const float2 *tw, const int *live = nullptr);
 // k_fft64.cu — FP64 transforms of any length n <= 4096 (k_fft64.cuh)
 bool fft64_any_supported(int n);
+bool fft64_smooth(int n);  // no prime factor above 7: transformed directly
+// exp(-2 pi i k / n), k < n, kept by the context.
+rg_status roots64(rg_context *ctx, int n, const double2 **out);
 // The context's plan for length n (its tables are made on the first call).
 rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out);
 // In-place 2-D transforms of `batch` ny x nx arrays.

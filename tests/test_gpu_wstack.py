@@ -26,6 +26,21 @@ def test_predict_matches_oracle(ctx, sim, oracle, lam, nv, npts, sw):
     assert np.linalg.norm(got - dft) / np.linalg.norm(dft) < 2e-3
 
 
+# few sources go directly, many (and supports above 16) through the stack: one
+# visibility or source, part-filled threads, every support class of the direct
+# path, a stack side that needs Bluestein's algorithm (412)
+@pytest.mark.parametrize("lam,nv,npts,suv,sw", [(1280.0, 1, 1, 8, 6), (1280.0, 257, 33, 8, 6), (1280.0, 500, 7, 6, 8),
+                                                (1280.0, 300, 65, 12, 4), (1280.0, 129, 5, 16, 16),
+                                                (1280.0, 200, 3, 18, 4), (1280.0, 30, 3000, 8, 6),
+                                                (2060.0, 50, 2000, 8, 4)])
+def test_predict_direct_and_stack_match_oracle(ctx, sim, oracle, lam, nv, npts, suv, sw):
+    c = case(sim, seed=nv + npts, lam=lam, nv=nv, npts=npts, suv=suv, sw=sw)
+    got = _run(ctx, c)
+    ref = oracle.wstack_predict(c["theta"], c["lam"], c["points"], c["u"], c["v"], c["w"], c["du"], c["dw"],
+                                c["x0"], c["conv_uv"], c["conv_w"], c["corr_lm"], c["corr_n"])
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-11
+
+
 def test_predict_device_buffers_and_errors(rg, ctx, sim):
     torch = pytest.importorskip("torch")
     c = case(sim, seed=5, nv=500)
