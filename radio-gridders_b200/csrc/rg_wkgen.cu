@@ -18,7 +18,8 @@
 // Xiao, Rokhlin & Yarvin 2001); the eigenvalue is found by Sturm-sequence
 // bisection and the eigenvector by inverse iteration (Wilkinson, The
 // Algebraic Eigenvalue Problem, ch. 5 and 9).  The screen and the two
-// non-uniform DFT sums run on the device in FP64.
+// non-uniform DFT sums run on the device in FP64, folded by the screen's
+// symmetry into real matrix products.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -147,80 +148,177 @@ double pswf_value(const std::vector<double> &coef, double x)
     return out / at0;
 }
 
-// s[plane][j][i] = A_i A_j exp(+2 pi i w (1 - n)), FP64.
+// The sums, folded. The screen is even in l and in m, so with i' = i - M/2 a
+// row's sum over i' = -M/2 .. M/2 - 1 is
+//   T(q) = s(0) + sum_{0 < i' < M/2} s(i') 2 cos(2 pi off_q i' / M) + s(-M/2) exp(pi i off_q),
+// real factors but for the unpaired edge, which takes two real columns of its
+// own: both sums are real matrix products of depth K = M/2 + 2 with one factor
+// matrix cq[k][q] = {1, 2 cos(2 pi off_q k / M), .., cos(pi off_q), sin(pi off_q)},
+// over M/2 + 2 rows j' in place of M. Off q = f*S + t (sub-cell shift f, tap t):
+// off_q = t - S/2 - f/ov.
+//
+// The products run on the FP64 tensor pipe (mma m8n8k4, 37 TFLOP/s measured, the
+// rate of the FP64 multiply-add pipe, with an eighth of its instructions and
+// operand reads): 64 x 64 tiles, K in shared memory 68 deep (all of the default
+// screen's 66), one 32 x 32 block a warp. Bound by that pipe: 2.6 GFLOP for
+// 401 planes of 16 x 16 taps, 8 x oversampled. The call: 4831 -> 374 us
+// (the sums as plain loops took 3387 and 1152 us).
+
+// a[k][row], row = (plane K + j') 2 + part: the screen's rows as the left
+// factor. k < M/2: s(i' = k); k = M/2, M/2 + 1: the edge i' = -M/2 times the
+// edge factors' real and imaginary parts. The rows j' run the same way, the
+// edge row twice, so the second product takes them as they come.
 __global__ void wscreen_kernel(const double *__restrict__ w_planes, int planes, const double *__restrict__ taper,
-                               int M, double theta, double2 *__restrict__ s)
+                               int M, double theta, double2 *__restrict__ a)
 {
-    const int64_t total = (int64_t)planes * M * M;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(k % M), j = (int)((k / M) % M), p = (int)(k / ((int64_t)M * M));
-        const double l = theta * (double)(i - M / 2) / M, m = theta * (double)(j - M / 2) / M;
+    const int h = M / 2, J = h + 1;
+    const int64_t pairs = (int64_t)planes * (h + 2), total = (int64_t)planes * J * J;
+    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < total; n += (int64_t)gridDim.x * blockDim.x) {
+        const int j = (int)(n % J), p = (int)((n / J) % planes), k = (int)(n / ((int64_t)J * planes));
+        const int ic = k < h ? k : -h, jc = j < h ? j : -h;
+        const double l = theta * (double)ic / M, m = theta * (double)jc / M;
         const double one_minus_n = 1.0 - sqrt(1.0 - (l * l + m * m));
         double sn, cs;
         sincospi(2.0 * w_planes[p] * one_minus_n, &sn, &cs);
-        const double a = taper[i] * taper[j];
-        s[k] = make_double2(a * cs, a * sn);
+        const double t = taper[ic + h] * taper[jc + h], re = t * cs, im = t * sn;
+        double2 *at = a + (int64_t)k * pairs + (int64_t)p * (h + 2) + j;
+        at[0] = make_double2(re, im);
+        if (k == h) at[pairs] = make_double2(-im, re);
+        if (j == h) {
+            at[1] = make_double2(-im, re);
+            if (k == h) at[pairs + 1] = make_double2(-re, -im);
+        }
     }
 }
 
-// E[q][i] = exp(-2 pi i off_q (i - M/2) / M), off_q = t - S/2 - f/ov for
-// q = f*S + t (sub-cell shift f, tap t).
-__global__ void wkgen_phasors_kernel(int S, int ov, int M, double2 *__restrict__ E)
+__global__ void wkgen_factors_kernel(int S, int ov, int M, double *__restrict__ cq)
 {
-    const int total = ov * S * M;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-        const int i = k % M, q = k / M;
-        const int f = q / S, t = q % S;
-        const double off = (double)(t - S / 2) - (double)f / ov;
-        double sn, cs;
-        sincospi(-2.0 * off * (double)(i - M / 2) / M, &sn, &cs);
-        E[k] = make_double2(cs, sn);
+    const int Q = ov * S, h = M / 2, total = Q * (h + 2);
+    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < total; n += gridDim.x * blockDim.x) {
+        const int q = n % Q, k = n / Q;
+        const double off = (double)(q % S - S / 2) - (double)(q / S) / ov;
+        cq[n] = k == 0 ? 1.0 : k < h ? 2.0 * cospi(2.0 * off * (double)k / M) : k == h ? cospi(off) : sinpi(off);
     }
 }
 
-__device__ __forceinline__ double2 cmad(double2 a, double2 b, double2 acc)
+constexpr int kGemmTile = 64, kGemmDepth = 68;
+constexpr int kGemmStride = kGemmTile + 4;  // 4 mod 16 doubles: a fragment's 4 k x 8 rows fall on distinct banks
+constexpr int kGemmThreads = 128;
+
+__device__ __forceinline__ void mma_f64(double2 &c, double a, double b)
 {
-    return make_double2(fma(a.x, b.x, fma(-a.y, b.y, acc.x)), fma(a.x, b.y, fma(a.y, b.x, acc.y)));
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c.x), "+d"(c.y)
+                 : "d"(a), "d"(b));
 }
 
-// T[plane][j][qx] = sum_i s[plane][j][i] E[qx][i]
-__global__ void wkgen_rows_kernel(const double2 *__restrict__ s, const double2 *__restrict__ E, int planes, int M,
-                                  int Q, double2 *__restrict__ T)
+// 16 bytes to shared memory, or zeros where !on
+__device__ __forceinline__ void cp_async16_if(void *smem, const void *gmem, bool on)
 {
-    const int64_t total = (int64_t)planes * M * Q;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const int qx = (int)(k % Q);
-        const int64_t pj = k / Q;  // plane * M + j
-        const double2 *row = s + pj * M;
-        const double2 *e = E + (int64_t)qx * M;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int i = 0; i < M; i++) acc = cmad(row[i], e[i], acc);
-        T[k] = acc;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+                 "l"(gmem), "r"(on ? 16 : 0)
+                 : "memory");
+}
+
+// One warp's 32 x 32 block of a 64 x 64 tile: rows row0 + 8 i, columns col(j) +
+// 0..7; c[i][j] holds row lane / 4, columns 2 (lane % 4) and the next. a and b
+// give a lane's two neighbouring elements of depth k (a warp copies one depth
+// of both), or nullptr past the edge.
+template <class A, class B, class Col>
+__device__ __forceinline__ void gemm_tile(double2 (&c)[4][4], double *sa, double *sb, int K, A a, B b, int row0, Col col)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k0 = 0; k0 < K; k0 += kGemmDepth) {
+        const int depth = min(kGemmDepth, (K - k0 + 3) & ~3);
+        __syncthreads();
+        for (int k = warp; k < depth; k += kGemmThreads / 32) {
+            const bool live = k0 + k < K;
+            const double *ga = live ? a(k0 + k, 2 * lane) : nullptr, *gb = live ? b(k0 + k, 2 * lane) : nullptr;
+            cp_async16_if(sa + k * kGemmStride + 2 * lane, ga, ga != nullptr);
+            cp_async16_if(sb + k * kGemmStride + 2 * lane, gb, gb != nullptr);
+        }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const double *pa = sa + (lane & 3) * kGemmStride + row0 + (lane >> 2);
+        const double *pb = sb + (lane & 3) * kGemmStride + (lane >> 2);
+        for (int k = 0; k < depth; k += 4) {
+            double fa[4], fb[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                fa[i] = pa[k * kGemmStride + 8 * i];
+                fb[i] = pb[k * kGemmStride + col(i)];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_f64(c[i][j], fa[i], fb[j]);
+        }
     }
 }
 
-// data[plane][yf][xf][ty][tx] = 1/M^2 sum_j E[qy][j] T[plane][j][qx],
-// qy = yf*S + ty, qx = xf*S + tx
-__global__ void wkgen_cols_kernel(const double2 *__restrict__ T, const double2 *__restrict__ E, int planes, int M,
-                                  int S, int ov, double2 *__restrict__ out)
+// T[row][qx] = sum_k a[k][row] cq[k][qx]
+__global__ void __launch_bounds__(kGemmThreads) wkgen_rows_kernel(const double *__restrict__ a,
+                                                                  const double *__restrict__ cq, int64_t rows, int K,
+                                                                  int Q, double *__restrict__ T)
 {
-    const int Q = ov * S;
-    const int64_t total = (int64_t)planes * Q * Q;
+    extern __shared__ double gemm_sm[];
+    const int64_t r0 = (int64_t)blockIdx.x * kGemmTile;
+    const int q0 = blockIdx.y * kGemmTile;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = (warp >> 1) * 32, col0 = (warp & 1) * 32;
+    double2 c[4][4] = {};
+    gemm_tile(
+        c, gemm_sm, gemm_sm + kGemmDepth * kGemmStride, K,
+        [&](int k, int x) { return r0 + x < rows ? a + k * rows + r0 + x : nullptr; },
+        [&](int k, int x) { return q0 + x < Q ? cq + (int64_t)k * Q + q0 + x : nullptr; }, row0,
+        [&](int j) { return col0 + 8 * j; });
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int64_t r = r0 + row0 + 8 * i + (lane >> 2);
+            const int q = q0 + col0 + 8 * j + 2 * (lane & 3);
+            if (r < rows && q < Q) {  // Q is even
+                *(double2 *)(T + r * Q + q) = c[i][j];
+            }
+        }
+}
+
+// data[plane][yf][xf][ty][tx] = 1/M^2 sum_k cq[k][qy] T[plane][k][part][qx],
+// qy = yf*S + ty, qx = xf*S + tx: 64 qy x 32 qx a tile, the imaginary parts
+// beside the real ones.
+__global__ void __launch_bounds__(kGemmThreads) wkgen_cols_kernel(const double *__restrict__ T,
+                                                                  const double *__restrict__ cq, int M, int S, int ov,
+                                                                  double2 *__restrict__ out)
+{
+    extern __shared__ double gemm_sm[];
+    const int Q = ov * S, h = M / 2, ytiles = (Q + kGemmTile - 1) / kGemmTile;
+    const int p = blockIdx.x / ytiles, y0 = (blockIdx.x % ytiles) * kGemmTile, x0 = blockIdx.y * 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = (warp >> 1) * 32, col0 = (warp & 1) * 16;
+    const double *Tp = T + (int64_t)p * (h + 2) * 2 * Q;
+    double2 c[4][4] = {};
+    gemm_tile(
+        c, gemm_sm, gemm_sm + kGemmDepth * kGemmStride, h + 2,
+        [&](int k, int x) { return y0 + x < Q ? cq + (int64_t)k * Q + y0 + x : nullptr; },
+        [&](int k, int x) {
+            const int part = x >> 5, q = x0 + (x & 31);
+            return q < Q ? Tp + ((int64_t)k * 2 + part) * Q + q : nullptr;
+        },
+        row0, [&](int j) { return col0 + 8 * (j & 1) + 32 * (j >> 1); });
     const double inv = 1.0 / ((double)M * M);
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        // output order [plane][yf][xf][ty][tx]
-        const int tx = (int)(k % S);
-        const int ty = (int)((k / S) % S);
-        const int xf = (int)((k / ((int64_t)S * S)) % ov);
-        const int yf = (int)((k / ((int64_t)S * S * ov)) % ov);
-        const int p = (int)(k / ((int64_t)Q * Q));
-        const int qx = xf * S + tx, qy = yf * S + ty;
-        const double2 *e = E + (int64_t)qy * M;
-        const double2 *t = T + (int64_t)p * M * Q + qx;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int j = 0; j < M; j++) acc = cmad(e[j], t[(int64_t)j * Q], acc);
-        out[k] = make_double2(acc.x * inv, acc.y * inv);
-    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int qy = y0 + row0 + 8 * i + (lane >> 2), qx = x0 + col0 + 8 * j + 2 * (lane & 3);
+            if (qy < Q && qx < Q) {
+                const int yf = qy / S, ty = qy - yf * S, xf = qx / S, tx = qx - xf * S;  // S is even
+                double2 *o = out + ((((int64_t)p * ov + yf) * ov + xf) * S + ty) * S + tx;
+                o[0] = make_double2(c[i][j].x * inv, c[i][j + 2].x * inv);
+                o[1] = make_double2(c[i][j].y * inv, c[i][j + 2].y * inv);
+            }
+        }
 }
 
 }  // namespace
@@ -264,24 +362,30 @@ rg_status rg_wkern_generate(rg_context *ctx, double theta, const double *w_plane
     for (int i = 0; i < M; i++) taper[i] = pswf_value(coef, 2.0 * (double)(i - M / 2) / M);
     const int S = size, ov = oversampling, Q = ov * S;
     const int64_t ntaps = (int64_t)plane_count * Q * Q;
-    void *d_w, *d_taper, *d_s, *d_E, *d_T;
+    const int J = M / 2 + 1, K = M / 2 + 2;
+    const int64_t rows = (int64_t)plane_count * K * 2;
+    void *d_w, *d_taper, *d_s, *d_cq, *d_T;
     RG_CHECK(scratch(ctx, "wkgen_w", sizeof(double) * plane_count, &d_w));
     RG_CHECK(scratch(ctx, "wkgen_taper", sizeof(double) * M, &d_taper));
-    RG_CHECK(scratch(ctx, "wkgen_screen", sizeof(double2) * (size_t)plane_count * M * M, &d_s));
-    RG_CHECK(scratch(ctx, "wkgen_phasors", sizeof(double2) * (size_t)Q * M, &d_E));
-    RG_CHECK(scratch(ctx, "wkgen_rows", sizeof(double2) * (size_t)plane_count * M * Q, &d_T));
+    RG_CHECK(scratch(ctx, "wkgen_screen", sizeof(double) * (size_t)rows * K, &d_s));
+    RG_CHECK(scratch(ctx, "wkgen_factors", sizeof(double) * (size_t)Q * K, &d_cq));
+    RG_CHECK(scratch(ctx, "wkgen_rows", sizeof(double) * (size_t)rows * Q, &d_T));
     OutView ov_out;
     RG_CHECK(out_view(ctx, data_out, sizeof(double2) * (size_t)ntaps, "wkgen_out", false, &ov_out));
     RG_CUDA(cudaMemcpyAsync(d_w, w_planes, sizeof(double) * plane_count, cudaMemcpyHostToDevice, ctx->stream));
     RG_CUDA(cudaMemcpyAsync(d_taper, taper.data(), sizeof(double) * M, cudaMemcpyHostToDevice, ctx->stream));
     auto blocks = [](int64_t n) { return (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 32); };
-    wscreen_kernel<<<blocks((int64_t)plane_count * M * M), 256, 0, ctx->stream>>>(
+    wscreen_kernel<<<blocks((int64_t)plane_count * J * J), 256, 0, ctx->stream>>>(
         (const double *)d_w, plane_count, (const double *)d_taper, M, theta, (double2 *)d_s);
-    wkgen_phasors_kernel<<<blocks((int64_t)Q * M), 256, 0, ctx->stream>>>(S, ov, M, (double2 *)d_E);
-    wkgen_rows_kernel<<<blocks((int64_t)plane_count * M * Q), 256, 0, ctx->stream>>>(
-        (const double2 *)d_s, (const double2 *)d_E, plane_count, M, Q, (double2 *)d_T);
-    wkgen_cols_kernel<<<blocks(ntaps), 256, 0, ctx->stream>>>((const double2 *)d_T, (const double2 *)d_E,
-                                                              plane_count, M, S, ov, (double2 *)ov_out.dev);
+    wkgen_factors_kernel<<<blocks((int64_t)Q * K), 256, 0, ctx->stream>>>(S, ov, M, (double *)d_cq);
+    const int smem = 2 * kGemmDepth * kGemmStride * (int)sizeof(double);
+    cudaFuncSetAttribute(wkgen_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(wkgen_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const unsigned tiles = (unsigned)((Q + kGemmTile - 1) / kGemmTile);
+    wkgen_rows_kernel<<<dim3((unsigned)((rows + kGemmTile - 1) / kGemmTile), tiles), kGemmThreads, smem, ctx->stream>>>(
+        (const double *)d_s, (const double *)d_cq, rows, K, Q, (double *)d_T);
+    wkgen_cols_kernel<<<dim3((unsigned)plane_count * tiles, (unsigned)((Q + 31) / 32)), kGemmThreads, smem,
+                        ctx->stream>>>((const double *)d_T, (const double *)d_cq, M, S, ov, (double2 *)ov_out.dev);
     ctx->launches += 4;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "w-kernel generator launch");

@@ -23,6 +23,19 @@ def test_generator_matches_python(ctx, sim, planes, size, ov):
         assert rel_rms(got[p], ref[p]) < 1e-12
 
 
+# one tap and many, tiles part filled, odd sub-cell counts, screens of one and
+# several depth chunks, the smallest screen; FP64 sums of up to 300 terms twice
+# (rounding below 1e-14), the tolerance of the test above
+@pytest.mark.parametrize("planes,size,ov,pixels", [([0.0], 2, 1, 4), ([3.0, -700.0], 6, 3, 10), ([50.0], 16, 5, 128),
+                                                   (list(range(-40, 41)), 4, 2, 128), ([-5.0, 9.5], 10, 7, 300),
+                                                   ([12.0], 64, 2, 136)])
+def test_generator_tile_edges_match_python(ctx, sim, planes, size, ov, pixels):
+    got = ctx.wkern_generate(0.1, np.array(planes), size, ov, c=9.0, screen_pixels=pixels)
+    ref = sim.generate_wkernel(0.1, np.array(planes, np.float64), size, ov, c=9.0, m_pix=pixels).data
+    for p in range(len(planes)):
+        assert rel_rms(got[p], ref[p]) < 1e-12
+
+
 def test_generated_table_grids_like_the_python_one(rg, ctx, sim, oracle):
     """A W-projection grid made with the generated table equals the oracle's
     with the Python table."""
