@@ -4,9 +4,11 @@
 // Both passes are bound by memory and by the latency of one CTA's
 // load - transform - store sequence, with the FP64 pipe behind them
 // (5 n^2 log2 n^2 operations: 0.7 GFLOP at n = 2500). One image of a 2500 x 2500
-// grid, with the caller's copy of the grid: 483 us, against 4522 us as
+// grid, with the caller's copy of the grid: 333 us, against 4522 us as
 // hermitian, shift, radix-2 Bluestein rows, transpose, rows, transpose, shift
-// and real part, each a pass of its own.
+// and real part, each a pass of its own. The rows take 114 us and the columns
+// 157 (193 and 227 with 16 points a thread and 11 warps an SM, strided
+// twiddles and addresses formed point by point).
 #include <algorithm>
 #include <string>
 
@@ -23,10 +25,11 @@ bool fft64_smooth(int n)
     return n == 1;
 }
 
-// Splits L into stages; false if it has a prime factor above 7. Powers of two
-// as 16s, the rest as one 8, 4 or 2, or as 8s where that leaves no 2; odd radices
+// Splits L into stages; false if it has a prime factor above 7. Odd radices
 // first: their first stage stores with an odd stride, free of bank conflicts.
-static bool fft64_stages(int L, Fft64Plan *p)
+// Powers of two as 8s (16s where a thread has the registers: wide) with one 4 or
+// 2 for the rest, or 4s in place of an 8 and a 2.
+static bool fft64_stages(int L, bool wide, Fft64Plan *p)
 {
     int n = L, lg = 0;
     p->nst = 0;
@@ -41,11 +44,14 @@ static bool fft64_stages(int L, Fft64Plan *p)
     }
     if (n != 1) return false;
     while (lg > 0) {
-        const int e = lg == 5 || lg == 6 || lg == 9 ? 3 : std::min(lg, 4);
+        int e = std::min(lg, 3);
+        if (wide) e = lg == 5 || lg == 6 || lg == 9 ? 3 : std::min(lg, 4);
+        else if (lg == 4) e = 2;
         p->radix[p->nst++] = 1 << e;
         lg -= e;
     }
     p->L = L;
+    p->pad = (L & (L - 1)) == 0 && L >= 256;
     int64_t ns = 1;
     for (int k = 0; k < p->nst; k++) {
         p->magic[k] = ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0u;
@@ -62,6 +68,17 @@ __global__ void fft64_twiddle_kernel(double2 *__restrict__ tw, int L)
     double s, c;
     sincospi(-2.0 * (double)k / (double)L, &s, &c);
     tw[k] = make_double2(c, s);
+}
+
+// One stage's twiddles: tw[i - 1][k] = exp(-2 pi i i k / (R Ns)), i < R, k < Ns.
+__global__ void fft64_stage_twiddle_kernel(double2 *__restrict__ tw, int R, int Ns)
+{
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= (R - 1) * Ns) return;
+    const int i = n / Ns + 1, k = n % Ns;
+    double s, c;
+    sincospi(-2.0 * (double)(i * k) / (double)(R * Ns), &s, &c);
+    tw[n] = make_double2(c, s);
 }
 
 // chirp[m] = exp(-pi i m^2 / n), the phase reduced exactly (m^2 mod 2n in
@@ -125,7 +142,7 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
     }
     Fft64Plan p;
     p.n = n;
-    bool direct = fft64_stages(n, &p);
+    const bool direct = fft64_stages(n, false, &p);
     if (!direct) {
         // the cheapest convolution length: points times passes over them, of
         // those whose stages fit one CTA's threads
@@ -133,7 +150,7 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
         int64_t cost = INT64_MAX;
         for (int L = 2 * n - 1; L <= 8192; L++) {
             Fft64Plan c;
-            if (!fft64_stages(L, &c) || fft64_threads(c, 0) > 512) continue;
+            if (!fft64_stages(L, true, &c) || fft64_threads<16>(c, 0) > 512) continue;
             if ((int64_t)L * (c.nst + 1) < cost) {
                 cost = (int64_t)L * (c.nst + 1);
                 best = c;
@@ -143,7 +160,15 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
         p.n = n;
     }
     p.scale = 1.0 / (double)p.L;
-    RG_CHECK(roots64(ctx, p.L, &p.tw));
+    void *tw;
+    RG_CHECK(scratch(ctx, ("fft64_" + std::to_string(n)).c_str(), sizeof(double2) * (size_t)p.L, &tw));
+    p.tw = (const double2 *)tw;
+    double2 *at = (double2 *)tw;
+    for (int k = 0, ns = 1; k < p.nst; ns *= p.radix[k++]) {
+        const int cnt = (p.radix[k] - 1) * ns;
+        if (k > 0) fft64_stage_twiddle_kernel<<<(cnt + 127) / 128, 128, 0, ctx->stream>>>(at, p.radix[k], ns);
+        at += cnt;
+    }
     if (!direct) {
         void *mem;
         RG_CHECK(scratch(ctx, ("chirp64_" + std::to_string(n)).c_str(), sizeof(double2) * (size_t)(p.L + n), &mem));

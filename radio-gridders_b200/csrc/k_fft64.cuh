@@ -193,106 +193,133 @@ __device__ __forceinline__ void static_for(F f)
     static_for_seq(f, std::make_integer_sequence<int, N>{});
 }
 
-// butterflies a thread holds at once: about 16 points in registers
-constexpr int fft64_per(int r) { return r == 16 ? 1 : r == 8 ? 2 : r == 7 ? 2 : r == 5 ? 3 : r == 4 ? 4 : r == 3 ? 5 : 4; }
-
-// Where point n of line t lies in the CTA's shared memory: lines one after
-// another, or interleaved for columns; one spare element after every 16 keeps
-// a stage's strided stores off one bank.
-template <bool COL>
-__device__ __forceinline__ int fft64_at(int t, int n, int L, int lgT)
+// Butterflies of radix r a thread holds at once, for about PTS points in registers.
+template <int PTS>
+__host__ __device__ constexpr int fft64_per(int r)
 {
-    const int a = COL ? (n << lgT) + t : t * L + n;
-    return a + (a >> 4);
+    return PTS / r > 1 ? PTS / r : 1;
 }
 
+// Threads of a CTA at most: 10 points a thread leave registers for 20 warps on an
+// SM, 16 points for 16.
+__host__ __device__ constexpr int fft64_max_threads(int pts) { return pts > 10 ? 512 : 640; }
+
+// Shared memory of a CTA: point n of line t at n + t L, or for columns
+// interleaved at n 2^lgT + t. With an odd first radix (every length that is not
+// a power of two) a stage's strided stores spread over the banks by themselves;
+// a power of two takes one spare element after every 16 (pad). Either way the
+// R points of a butterfly lie at one stride from its first.
 struct Fft64Work {
     double2 *sm;
     int L, lgT;
+    bool pad;
 };
 
 // One Stockham stage of radix R: sub-transforms of length Ns become R Ns long.
+// tw: the stage's twiddles exp(-2 pi i i k / (R Ns)) at [i - 1][k], k < Ns.
 // from_in: points come from in(t, n); to_out: results go to out(t, n, v).
 // filter: a result in shared memory is multiplied by filter[n] and its parts
 // exchanged (the inverse transform follows as a forward one).
-template <int R, bool COL, class In, class Out>
+template <int R, int PTS, bool COL, class In, class Out>
 __device__ __forceinline__ void fft64_stage(const Fft64Work &w, const double2 *__restrict__ tw, int Ns,
                                             unsigned magic, bool from_in, bool to_out,
                                             const double2 *__restrict__ filter, In in, Out out)
 {
-    constexpr int PER = fft64_per(R);
+    constexpr int PER = fft64_per<PTS>(R);
     // opaque to the compiler, which would otherwise compute every radix's
     // addresses ahead of the stage loop and spill them
     int L = w.L;
     asm volatile("" : "+r"(L));
-    const int nj = L / R, items = nj << w.lgT, tstep = nj / Ns;
+    const int nj = L / R, items = nj << w.lgT, lg = COL ? w.lgT : 0;
+    const int ld = nj << lg, lds = ld + (w.pad ? ld >> 4 : 0);  // a butterfly's stride when read
     double2 a[PER][R];
+    int line[PER], first[PER], block[PER];  // a butterfly's line, its j and j / Ns * Ns
+    // a thread past the last butterfly repeats it and stores nothing: the
+    // registers are written on every path, so none live from stage to stage
     static_for<PER>([&](auto q) {
-        // a thread past the last butterfly repeats it and stores nothing: the
-        // registers are written on every path, so none live from stage to stage
         const int it = min((int)(threadIdx.x + q * blockDim.x), items - 1);
-        const int t = COL ? it & ((1 << w.lgT) - 1) : it / nj, j = COL ? it >> w.lgT : it - t * nj;
-        if (from_in) {
-            static_for<R>([&](auto i) { a[q][i] = in(t, j + i * nj); });
-        } else {
-            static_for<R>([&](auto i) { a[q][i] = w.sm[fft64_at<COL>(t, j + i * nj, L, w.lgT)]; });
-            if (Ns > 1) {
-                const int k = (j - (int)__umulhi((unsigned)j, magic) * Ns) * tstep;
-                static_for<R - 1>([&](auto i) { a[q][i + 1] = cmul64(a[q][i + 1], __ldg(tw + (i + 1) * k)); });
-            }
-        }
-        Dft64<R>::run(a[q]);
+        const int t = COL ? it & ((1 << w.lgT) - 1) : w.lgT ? it / nj : 0;
+        const int j = COL ? it >> w.lgT : it - t * nj;
+        line[q] = t;
+        first[q] = j;
+        block[q] = Ns > 1 ? (int)__umulhi((unsigned)j, magic) * Ns : j;
     });
+    if (from_in) {
+        static_for<PER>([&](auto q) { static_for<R>([&](auto i) { a[q][i] = in(line[q], first[q] + i * nj); }); });
+    } else {
+        static_for<PER>([&](auto q) {
+            const int n = COL ? (first[q] << lg) + line[q] : first[q] + line[q] * L;
+            const double2 *src = w.sm + n + (w.pad ? n >> 4 : 0);
+            static_for<R>([&](auto i) { a[q][i] = src[i * lds]; });
+            if (Ns > 1) {
+                const double2 *wk = tw + (first[q] - block[q]);
+                static_for<R - 1>([&](auto i) { a[q][i + 1] = cmul64(a[q][i + 1], __ldg(wk + i * Ns)); });
+            }
+        });
+    }
+    static_for<PER>([&](auto q) { Dft64<R>::run(a[q]); });
     if (!to_out) __syncthreads();  // every read of this stage is done
     static_for<PER>([&](auto q) {
-        const int it = threadIdx.x + q * blockDim.x;
-        if (it < items) {
-            const int t = COL ? it & ((1 << w.lgT) - 1) : it / nj, j = COL ? it >> w.lgT : it - t * nj;
-            const int b = Ns > 1 ? (int)__umulhi((unsigned)j, magic) * Ns : j;
-            const int d0 = b * R + (j - b);
-            static_for<R>([&](auto i) {
-                const int d = d0 + i * Ns;
-                if (to_out) out(t, d, a[q][i]);
-                else w.sm[fft64_at<COL>(t, d, L, w.lgT)] = filter ? swap64(cmul64(a[q][i], __ldg(filter + d))) : a[q][i];
-            });
+        if ((int)(threadIdx.x + q * blockDim.x) < items) {
+            const int d0 = block[q] * R + (first[q] - block[q]);
+            if (to_out) {
+                static_for<R>([&](auto i) { out(line[q], d0 + i * Ns, a[q][i]); });
+            } else {
+                if (filter)
+                    static_for<R>([&](auto i) { a[q][i] = swap64(cmul64(a[q][i], __ldg(filter + d0 + i * Ns))); });
+                const int n = COL ? (d0 << lg) + line[q] : d0 + line[q] * L, step = Ns << lg;
+                double2 *dst = w.sm + n;
+                if (w.pad) {
+                    // n's place in its 16 is below step, or step is a multiple of 16
+                    dst += n >> 4;
+                    static_for<R>([&](auto i) { dst[i * step + ((i * step) >> 4)] = a[q][i]; });
+                } else {
+                    static_for<R>([&](auto i) { dst[i * step] = a[q][i]; });
+                }
+            }
         }
     });
     if (!to_out) __syncthreads();
 }
 
-template <bool COL, class In, class Out>
+template <int PTS, bool COL, class In, class Out>
 __device__ __forceinline__ void fft64_transform(const Fft64Work &w, const Fft64Plan &p, bool first_in, bool last_out,
                                                 const double2 *filter, In in, Out out)
 {
     int Ns = 1;
+    const double2 *tw = p.tw;
 #pragma unroll 1
     for (int s = 0; s < p.nst; s++) {
         const bool fi = first_in && s == 0, last = s + 1 == p.nst, lo = last_out && last;
         const double2 *f = last ? filter : nullptr;
         const unsigned mg = p.magic[s];
-        switch (p.radix[s]) {
-            case 16: fft64_stage<16, COL>(w, p.tw, Ns, mg, fi, lo, f, in, out); break;
-            case 8: fft64_stage<8, COL>(w, p.tw, Ns, mg, fi, lo, f, in, out); break;
-            case 7: fft64_stage<7, COL>(w, p.tw, Ns, mg, fi, lo, f, in, out); break;
-            case 5: fft64_stage<5, COL>(w, p.tw, Ns, mg, fi, lo, f, in, out); break;
-            case 4: fft64_stage<4, COL>(w, p.tw, Ns, mg, fi, lo, f, in, out); break;
-            case 3: fft64_stage<3, COL>(w, p.tw, Ns, mg, fi, lo, f, in, out); break;
-            default: fft64_stage<2, COL>(w, p.tw, Ns, mg, fi, lo, f, in, out); break;
+        const int r = p.radix[s];
+        switch (r) {
+            case 16:
+                if constexpr (PTS >= 16) fft64_stage<16, PTS, COL>(w, tw, Ns, mg, fi, lo, f, in, out);
+                break;
+            case 8: fft64_stage<8, PTS, COL>(w, tw, Ns, mg, fi, lo, f, in, out); break;
+            case 7: fft64_stage<7, PTS, COL>(w, tw, Ns, mg, fi, lo, f, in, out); break;
+            case 5: fft64_stage<5, PTS, COL>(w, tw, Ns, mg, fi, lo, f, in, out); break;
+            case 4: fft64_stage<4, PTS, COL>(w, tw, Ns, mg, fi, lo, f, in, out); break;
+            case 3: fft64_stage<3, PTS, COL>(w, tw, Ns, mg, fi, lo, f, in, out); break;
+            default: fft64_stage<2, PTS, COL>(w, tw, Ns, mg, fi, lo, f, in, out); break;
         }
-        Ns *= p.radix[s];
+        tw += (r - 1) * Ns;
+        Ns *= r;
     }
 }
 
 // CTA = 2^lgT lines of one array (`lines` lines an array, `groups` CTAs an
 // array). ld(array, line, n) and st(array, line, n, v) move the points; swap:
 // the backward transform (parts exchanged on the way in and out).
-template <bool COL, bool BLUESTEIN, class Ld, class St>
-__global__ void __launch_bounds__(512) fft64_lines_kernel(Fft64Plan p, int lines, int groups, int lgT, bool swap, Ld ld,
+template <int PTS, bool COL, bool BLUESTEIN, class Ld, class St>
+__global__ void __launch_bounds__(fft64_max_threads(PTS)) fft64_lines_kernel(Fft64Plan p, int lines, int groups, int lgT, bool swap, Ld ld,
                                                           St st)
 {
     extern __shared__ double2 fft64_sm[];
     const int arr = blockIdx.x / groups, line0 = (blockIdx.x % groups) << lgT;
-    Fft64Work w{fft64_sm, p.L, lgT};
+    const Fft64Work w{fft64_sm, p.L, lgT, p.pad};
     auto in = [&](int t, int n) -> double2 {
         double2 v = make_double2(0.0, 0.0);
         if (line0 + t < lines && (!BLUESTEIN || n < p.n)) {
@@ -311,19 +338,20 @@ __global__ void __launch_bounds__(512) fft64_lines_kernel(Fft64Plan p, int lines
         st(arr, line0 + t, n, swap ? swap64(v) : v);
     };
     if (BLUESTEIN) {
-        fft64_transform<COL>(w, p, true, false, p.filter, in, out);
-        fft64_transform<COL>(w, p, false, true, nullptr, in, out);
+        fft64_transform<PTS, COL>(w, p, true, false, p.filter, in, out);
+        fft64_transform<PTS, COL>(w, p, false, true, nullptr, in, out);
     } else {
-        fft64_transform<COL>(w, p, true, true, nullptr, in, out);
+        fft64_transform<PTS, COL>(w, p, true, true, nullptr, in, out);
     }
 }
 
 // Threads for 2^lgT lines: enough for every stage's butterflies at once.
-inline int fft64_threads(const Fft64Plan &p, int lgT)
+template <int PTS>
+int fft64_threads(const Fft64Plan &p, int lgT)
 {
     int threads = 32;
     for (int k = 0; k < p.nst; k++) {
-        const int items = (p.L / p.radix[k]) << lgT, per = fft64_per(p.radix[k]);
+        const int items = (p.L / p.radix[k]) << lgT, per = fft64_per<PTS>(p.radix[k]);
         threads = threads > (items + per - 1) / per ? threads : (items + per - 1) / per;
     }
     return (threads + 31) & ~31;
@@ -335,7 +363,7 @@ inline int fft64_threads(const Fft64Plan &p, int lgT)
 // 32-byte sector is read once.
 inline int fft64_lines_lg(const Fft64Plan &p, bool col, int64_t lines)
 {
-    auto fits = [&](int lg) { return (p.L << lg) <= (col ? 8192 : 2048) && fft64_threads(p, lg) <= 512; };
+    auto fits = [&](int lg) { return (p.L << lg) <= (col ? 8192 : 2048) && fft64_threads<16>(p, lg) <= 512; };
     int lg = 0;
     while (lg < (col ? 3 : 2) && fits(lg + 1) && (lines >> (lg + 1)) >= 2 * 148) lg++;
     if (col && lg == 0 && lines > 1 && fits(1)) lg = 1;
@@ -349,14 +377,19 @@ void launch_fft64_lines(cudaStream_t s, const Fft64Plan &p, int batch, int lines
     const int lgT = fft64_lines_lg(p, COL, (int64_t)batch * lines);
     const int groups = (lines + (1 << lgT) - 1) >> lgT;
     const int pts = p.L << lgT;
-    const size_t smem = p.nst < 2 && !p.chirp ? 0 : sizeof(double2) * (size_t)(pts + pts / 16 + 1);
-    const int threads = fft64_threads(p, lgT);
-    auto go = [&](auto kernel) {
+    const size_t smem = p.nst < 2 && !p.chirp ? 0 : sizeof(double2) * (size_t)(pts + (p.pad ? pts / 16 : 0));
+    auto go = [&](auto kernel, int threads) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kernel<<<(unsigned)batch * groups, threads, smem, s>>>(p, lines, groups, lgT, sign > 0, ld, st);
     };
-    if (p.chirp) go(fft64_lines_kernel<COL, true, Ld, St>);
-    else go(fft64_lines_kernel<COL, false, Ld, St>);
+    // 10 points a thread for more warps on an SM; 16 where that would need too
+    // many threads and for the convolution lengths' radix 16
+    bool wide = false;
+    for (int k = 0; k < p.nst; k++) wide = wide || p.radix[k] > 8;
+    const int few = fft64_threads<10>(p, lgT);
+    if (p.chirp) go(fft64_lines_kernel<16, COL, true, Ld, St>, fft64_threads<16>(p, lgT));
+    else if (!wide && few <= fft64_max_threads(10)) go(fft64_lines_kernel<10, COL, false, Ld, St>, few);
+    else go(fft64_lines_kernel<16, COL, false, Ld, St>, fft64_threads<16>(p, lgT));
 }
 
 }  // namespace rg

@@ -94,9 +94,10 @@ namespace rg {
 // the convolution length of Bluestein's algorithm (chirp and filter set).
 struct Fft64Plan {
     int n = 0, L = 0, nst = 0;
+    bool pad = false;         // L is a power of two: padded in shared memory
     int radix[12] = {};       // the stages' radices
     unsigned magic[12] = {};  // ceil(2^32 / Ns): a stage's j / Ns by one high multiply
-    const double2 *tw = nullptr;      // exp(-2 pi i k / L), k < L
+    const double2 *tw = nullptr;      // the stages' twiddles, one after another (below L in all)
     const double2 *chirp = nullptr;   // exp(-pi i m^2 / n), m < n
     const double2 *filter = nullptr;  // transform of the wrapped conj(chirp), L points
     double scale = 1.0;               // 1 / L

@@ -342,17 +342,17 @@ rg_status host_table(const rg_sepkern *k, std::vector<double> &hold, const doubl
 // Direct: 0.103 ps a source, visibility and multiply-add (512 us for 400
 // sources x 200,000 visibilities at supports 8, 8, 6), but 0.37 us a source at
 // least, the time of one CTA's step, when the visibilities are too few to fill
-// the device. Stack: 25 ps a cell and plane (1543 us for 15 planes of 2048 x
-// 2048 cells), 160 ps where G needs Bluestein's algorithm, and 5 ps a tap
-// (383 us for 200,000 x 384). 50 sources and 200,000 visibilities: 88 us
-// against 1.9 ms; 20,000 sources: 26 ms against 1.9 ms.
+// the device. Stack: 23 ps a cell and plane (1444 us for 15 planes of 2048 x
+// 2048 cells), 106 ps where G needs Bluestein's algorithm (6747 us at 2060), and
+// 5 ps a tap (383 us for 200,000 x 384). 50 sources and 200,000 visibilities:
+// 88 us against 1.8 ms; 20,000 sources: 26 ms against 1.8 ms.
 bool wstack_use_direct(int64_t nvis, int nsrc, int planes, int G, int suv, int sw)
 {
     if (suv > 16 || sw > 16) return false;
     const bool wide = suv > 8 || sw > 8;
     const double fma = 2.0 * (wide ? 48 : 16 + (sw <= 6 ? 6 : 8)) + 18;
     const double direct = nsrc * std::max((double)nvis * fma * 0.103e-12, 0.37e-6);
-    const double cell = fft64_smooth(G) ? 25e-12 : 160e-12;
+    const double cell = fft64_smooth(G) ? 23e-12 : 106e-12;
     const double stack = (double)planes * G * G * cell + (double)nvis * suv * suv * sw * 5e-12;
     return direct <= stack;
 }
