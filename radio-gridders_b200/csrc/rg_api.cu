@@ -1383,8 +1383,14 @@ rg_status rg_dft_image_rows(rg_context *ctx, double *image_out, int grid_size, d
     RG_CHECK(stage_vis(ctx, vis, &dv));
     OutView ov;
     RG_CHECK(out_view(ctx, image_out, sizeof(double) * (size_t)nrows * grid_size, "dft_out", false, &ov));
+    void *work = nullptr;
+    if (precision == RG_DFT_FP64) {
+        const size_t shares = dft64_shares(grid_size, dv.n, ctx->sm_count);
+        const size_t part = shares > 1 ? shares * nrows * grid_size : 0;
+        RG_CHECK(scratch(ctx, "dft64_work", sizeof(double) * (2 + part), &work));
+    }
     launch_dft(ctx->stream, dv.u, dv.v, dv.w, dv.vis, dv.n, (double *)ov.dev, grid_size, theta, precision,
-               factor, ctx->sm_count, row0, nrows);
+               factor, ctx->sm_count, row0, nrows, (double *)work);
     RG_CHECK(check_launch("dft"));
     RG_CHECK(finish_out(ctx, ov));
     RG_CUDA(cudaStreamSynchronize(ctx->stream));

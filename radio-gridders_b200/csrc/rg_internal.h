@@ -348,7 +348,11 @@ void launch_add_back(cudaStream_t s, const float2 *subimg, const int *tower_coun
 // nrows < 0: the whole image
 void launch_dft(cudaStream_t s, const double *u, const double *v, const double *w,
                 const double2 *vis, int64_t n, double *image, int grid_size, double theta,
-                int precision, double factor, int sm_count, int row0 = 0, int nrows = -1);
+                int precision, double factor, int sm_count, int row0 = 0, int nrows = -1,
+                double *work = nullptr);
+// Shares of the visibilities in the FP64 mode, whose work space is 2 doubles,
+// and shares * nrows * grid_size more if there are several.
+int dft64_shares(int grid_size, int64_t n, int sm_count);
 
 // k_mlp.cu — learned w-kernel
 int mlp_param_count();

@@ -122,6 +122,52 @@ def test_dft_precision_modes(rg, ctx, oracle, dft_case):
     assert err[rg.RG_DFT_FP64_REDUCED] < err[rg.RG_DFT_FP32_NAIVE]
 
 
+def _dft64_numpy(n, th, u, v, w, vis):
+    lm = th * (np.arange(n) - n // 2) / n
+    out = np.empty((n, n))
+    with np.errstate(invalid="ignore"):
+        for y in range(n):
+            ph = np.outer(lm, u) + lm[y] * v + np.outer(1 - np.sqrt(1 - lm * lm - lm[y] ** 2), w)
+            ph -= np.round(ph)
+            out[y] = 2 * (np.cos(2 * np.pi * ph) @ vis.real + np.sin(2 * np.pi * ph) @ vis.imag)
+    return out
+
+
+# tiles part filled, odd counts, one moment (w = 0) to eight, more than eight (the
+# per-pixel kernel), pixels beyond the horizon, one share of the visibilities and
+# several. Phases of up to 500 turns are rounded three times (1e-16 relative
+# each): 1e-12 of the image's peak covers it.
+@pytest.mark.parametrize("n,nv,th,wmax", [(1, 1, 0.1, 10.0), (32, 31, 0.05, 0.0), (33, 3001, 0.05, 500.0),
+                                          (97, 1203, 0.1, 2000.0), (64, 1000, 0.1, 2000.0), (50, 700, 0.4, 2000.0),
+                                          (200, 640, 0.02, 5.0), (40, 200, 1.5, 50.0), (96, 333, 1.2, 1.0)])
+def test_dft_fp64_tiles_vs_numpy(rg, ctx, n, nv, th, wmax):
+    rng = np.random.default_rng(n + nv)
+    u, v = rng.uniform(-0.5 * n / th, 0.5 * n / th, (2, nv))
+    w = rng.uniform(-wmax, wmax, nv)
+    vis = rng.normal(size=nv) + 1j * rng.normal(size=nv)
+    V = rg.Visibilities(u, v, w, vis)
+    img = ctx.dft_image(n, th, V, rg.RG_DFT_FP64, 2.0)
+    ref = _dft64_numpy(n, th, u, v, w, vis)
+    assert np.array_equal(np.isnan(img), np.isnan(ref))
+    assert np.nanmax(np.abs(img - ref)) < 1e-12 * np.nanmax(np.abs(ref))
+    if n > 32:  # a band that starts on a tile is the whole image's rows
+        assert np.array_equal(ctx.dft_image_rows(n, th, V, 32, n - 32, rg.RG_DFT_FP64), img[32:], equal_nan=True)
+
+
+def test_dft_fp64_non_finite_and_empty_inputs(rg, ctx):
+    n, th = 40, 0.1
+    u, v, w = np.array([10.0, 20.0]), np.array([-5.0, 3.0]), np.array([1.0, 2.0])
+    vis = np.array([1.0 + 0j, np.inf + 0j])
+    img = ctx.dft_image(n, th, rg.Visibilities(u, v, w, vis), rg.RG_DFT_FP64, 2.0)
+    assert not np.isfinite(img).any()
+    w[1] = np.nan
+    img = ctx.dft_image(n, th, rg.Visibilities(u, v, w, np.ones(2, complex)), rg.RG_DFT_FP64, 2.0)
+    assert np.isnan(img).all()
+    e = np.zeros(0)
+    img = ctx.dft_image(n, th, rg.Visibilities(e, e, e, np.zeros(0, complex)), rg.RG_DFT_FP64, 2.0)
+    assert np.array_equal(img, np.zeros((n, n)))
+
+
 def test_dft_single_visibility_fringe(rg, ctx):
     n, th = 64, 0.1
     u, v, w = np.array([37.0]), np.array([-12.0]), np.array([3.0])
