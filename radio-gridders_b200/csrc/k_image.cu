@@ -22,28 +22,10 @@ __global__ void convert_table_kernel(const double2 *__restrict__ src, float2 *__
     }
 }
 
-void launch_convert_table(cudaStream_t s, const double2 *src, float2 *dst, int64_t n)
-{
-    convert_table_kernel<<<blocks_for(n), 256, 0, s>>>(src, dst, n);
-}
-
-// Each kk-tap slice written twice in a row: dst[s][0..2kk) = src[s][t mod kk].
-__global__ void convert_table_dup_kernel(const double2 *__restrict__ src, float2 *__restrict__ dst, int64_t n_out,
-                                         int kk)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_out;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t slice = i / (2 * kk);
-        const double2 z = src[slice * kk + (int)(i % (2 * kk)) % kk];
-        dst[i] = make_float2((float)z.x, (float)z.y);
-    }
-}
-
-// The same for a power-of-two slice length (every supported kernel size): one
-// thread per two source taps (two 16-byte loads), each converted pair stored
-// twice as one 16-byte store; shifts instead of 64-bit divisions.
-__global__ void convert_table_dup_pow2_kernel(const double2 *__restrict__ src, float4 *__restrict__ dst,
-                                              int64_t n_pairs, int kk_lg)
+// Each K x K slice written twice in a row: one thread per two source
+// taps (two 16-byte loads), each converted pair stored twice as one 16-byte store.
+__global__ void convert_table_dup_kernel(const double2 *__restrict__ src, float4 *__restrict__ dst,
+                                         int64_t n_pairs, int kk_lg)
 {
     const int64_t half = (int64_t)1 << (kk_lg - 1);  // pairs per slice
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_pairs;
@@ -57,14 +39,27 @@ __global__ void convert_table_dup_pow2_kernel(const double2 *__restrict__ src, f
     }
 }
 
-void launch_convert_table_dup(cudaStream_t s, const double2 *src, float2 *dst, int64_t n, int kk)
+// The paired layout (K 16 or 32): entry i = [r][c] of a slice, r < K/2, from the
+// taps of rows r and r + K/2, half a slice apart.
+__global__ void convert_table_pairs_kernel(const double2 *__restrict__ src, float4 *__restrict__ dst,
+                                           int64_t n_pairs, int kk_lg)
+{
+    const int64_t half = (int64_t)1 << (kk_lg - 1);  // entries per slice
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_pairs;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const double2 *s = src + ((i >> (kk_lg - 1)) << kk_lg) + (i & (half - 1));
+        const double2 a = s[0], b = s[half];
+        dst[i] = make_float4((float)a.x, (float)b.x, (float)a.y, (float)b.y);
+    }
+}
+
+void launch_convert_taps(cudaStream_t s, const double2 *src, float2 *dst, int64_t n, int ksize, bool strips)
 {
     int lg = 0;
-    while ((1 << lg) < kk) lg++;
-    if ((1 << lg) == kk && lg >= 1)
-        convert_table_dup_pow2_kernel<<<blocks_for(n / 2), 256, 0, s>>>(src, (float4 *)dst, n / 2, lg);
-    else
-        convert_table_dup_kernel<<<blocks_for(2 * n), 256, 0, s>>>(src, dst, 2 * n, kk);
+    while ((1 << lg) < ksize * ksize) lg++;
+    if (strips) convert_table_dup_kernel<<<blocks_for(n / 2), 256, 0, s>>>(src, (float4 *)dst, n / 2, lg);
+    else if (ksize >= 16) convert_table_pairs_kernel<<<blocks_for(n / 2), 256, 0, s>>>(src, (float4 *)dst, n / 2, lg);
+    else convert_table_kernel<<<blocks_for(n), 256, 0, s>>>(src, dst, n);
 }
 
 // make_hermitian, src/reference/grid.c:639-662: the pointer walk pairs linear

@@ -29,6 +29,9 @@
 // Visibilities are staged through shared memory in batches (coalesced 16-byte
 // record and 8-byte visibility loads); taps are read through the read-only
 // cache, one oversampled K x K slice per visibility.
+//
+// romein_pairs_kernel serves row-major grids with converted tables of 16 and 32
+// cells, romein_kernel the rest.
 #include "rg_internal.h"
 
 namespace rg {
@@ -188,37 +191,179 @@ __global__ void __launch_bounds__(K *K / P, (RomeinBounds<K, P>::min_ctas)) rome
     }
 }
 
+// Row-major grids, supports of 16 and 32, with a converted table in the paired
+// layout (launch_convert_table_pairs): entry [r][c], r < K/2, of a slice holds the
+// taps of rows r and r + K/2 as (re, re, im, im). A thread's points are taken in
+// pairs K/2 rows apart, so one 16-byte load brings both taps ready for packed
+// multiply-adds whose other operands, (re, re), (im, im) and (-re, -re) of the
+// visibility, come from shared memory: per tap two issue slots and no packing,
+// with the roundings of the form above. Which point of a pair lies in the lower
+// half of the slice depends on the footprint's row; where that turns over, the
+// pair's sums and keys are exchanged.
+// Bound by instruction issue and the latency of the taps' loads from L2: 213 us
+// for 1,000,000 visibilities on 2048 x 2048 (16 cells), 265 us with a point's taps
+// loaded one by one and packed. The strip-major sub-grids keep the form above:
+// there the pairs' turning over costs more (526 -> 720 us on 2.09 M visibilities).
+template <int K, int P>
+__global__ void __launch_bounds__(K *K / P, (RomeinBounds<K, P>::min_ctas)) romein_pairs_kernel(
+    const int4 *__restrict__ rec, const float2 *__restrict__ visf, int64_t n, const float4 *__restrict__ taps,
+    float2 *__restrict__ grids, const int *__restrict__ slot_of_bin, int64_t grid_stride, int side, int64_t chunk,
+    int slot_cap)
+{
+    constexpr int NT = K * K / P;  // threads
+    constexpr int BATCH = 128;     // visibilities staged per round
+    constexpr int RS = K / P;      // row stride between a thread's points
+    constexpr int H = P / 2, KH = K / 2;
+    __shared__ int4 srec[BATCH];
+    __shared__ float4 svis[BATCH];   // (re, re, im, im)
+    __shared__ float2 snre[BATCH];   // (-re, -re)
+    const int myU = threadIdx.x % K, myV0 = threadIdx.x / K;
+    for (int64_t c0 = (int64_t)blockIdx.x * chunk; c0 < n; c0 += (int64_t)gridDim.x * chunk) {
+        const int64_t c1 = c0 + chunk < n ? c0 + chunk : n;
+        int cur_bin = -1, cur_goff = 0, cur_res = 0;
+        float2 *cur_grid = nullptr;  // the current bin's sub-grid (null: past the slot capacity)
+        int key_lo[H], key_hi[H];    // element offsets of the pairs' points, -1 off the grid
+        float2 re[H], im[H];         // (lower point, upper point)
+#pragma unroll
+        for (int q = 0; q < H; q++) {
+            key_lo[q] = key_hi[q] = -1;
+            re[q] = im[q] = make_float2(0.f, 0.f);
+        }
+        auto flush_lo = [&](int q) {
+            if (cur_grid && key_lo[q] >= 0) atomicAdd(cur_grid + key_lo[q], make_float2(re[q].x, im[q].x));
+        };
+        auto flush_hi = [&](int q) {
+            if (cur_grid && key_hi[q] >= 0) atomicAdd(cur_grid + key_hi[q], make_float2(re[q].y, im[q].y));
+        };
+        for (int64_t b0 = c0; b0 < c1; b0 += BATCH) {
+            const int cnt = (int)(c1 - b0 < BATCH ? c1 - b0 : BATCH);
+            __syncthreads();
+            for (int j = threadIdx.x; j < cnt; j += NT) {
+                srec[j] = rec[b0 + j];
+                const float2 z = visf[b0 + j];
+                svis[j] = make_float4(z.x, z.x, z.y, z.y);
+                snre[j] = make_float2(-z.x, -z.x);
+            }
+            __syncthreads();
+            for (int j = 0; j < cnt; j++) {
+                const int4 r = srec[j];
+                if (r.x < 0) continue;
+                const int cu = (myU - (r.w & 0xff)) & (K - 1);
+                // slice row of the thread's first point
+                const int cv0 = (myV0 - (r.w >> 16)) & (K - 1);
+                const float4 *tp = taps + (int64_t)(r.z >> 1) + cu;
+                float4 t[H];
+#pragma unroll
+                for (int q = 0; q < H; q++) t[q] = __ldg(tp + ((cv0 + q * RS) & (KH - 1)) * K);
+                const float4 vz = svis[j];
+                const float2 vre = make_float2(vz.x, vz.y), vim = make_float2(vz.z, vz.w), nre = snre[j];
+                if (!(r.x == cur_bin && r.y == cur_goff && r.w == cur_res)) {
+                    cur_goff = r.y;
+                    cur_res = r.w;
+                    int lo[H], hi[H];
+                    // per-axis check; -1 (never flushed) for a tap off the grid
+                    const int col = (r.w & 0xffff) - 64 + cu;
+                    const int row0 = (r.w >> 16) - 64;
+                    const bool in_col = (unsigned)col < (unsigned)side;
+#pragma unroll
+                    for (int q = 0; q < H; q++) {
+                        const int row = row0 + ((cv0 + q * RS) & (KH - 1));
+                        lo[q] = in_col && (unsigned)row < (unsigned)side ? row * side + col : -1;
+                        hi[q] = in_col && (unsigned)(row + KH) < (unsigned)side ? (row + KH) * side + col : -1;
+                    }
+                    if (r.x != cur_bin) {
+#pragma unroll
+                        for (int q = 0; q < H; q++) {
+                            flush_lo(q);
+                            flush_hi(q);
+                            key_lo[q] = lo[q];
+                            key_hi[q] = hi[q];
+                            re[q] = im[q] = make_float2(0.f, 0.f);
+                        }
+                        cur_bin = r.x;
+                        const int slot = slot_of_bin[cur_bin];
+                        cur_grid = slot < slot_cap ? grids + (int64_t)slot * grid_stride : nullptr;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < H; q++) {
+                            if (lo[q] == key_lo[q] && hi[q] == key_hi[q]) continue;
+                            if (lo[q] == key_hi[q] || hi[q] == key_lo[q]) {  // the halves turned over
+                                const int k = key_lo[q];
+                                key_lo[q] = key_hi[q];
+                                key_hi[q] = k;
+                                re[q] = make_float2(re[q].y, re[q].x);
+                                im[q] = make_float2(im[q].y, im[q].x);
+                            }
+                            if (lo[q] != key_lo[q]) {
+                                flush_lo(q);
+                                key_lo[q] = lo[q];
+                                re[q].x = im[q].x = 0.f;
+                            }
+                            if (hi[q] != key_hi[q]) {
+                                flush_hi(q);
+                                key_hi[q] = hi[q];
+                                re[q].y = im[q].y = 0.f;
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < H; q++) {
+                    const float2 tx = make_float2(t[q].x, t[q].y), ty = make_float2(t[q].z, t[q].w);
+                    re[q] = __ffma2_rn(ty, vim, re[q]);
+                    im[q] = __ffma2_rn(ty, nre, im[q]);
+                    re[q] = __ffma2_rn(tx, vre, re[q]);
+                    im[q] = __ffma2_rn(tx, vim, im[q]);
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < H; q++) {
+            flush_lo(q);
+            flush_hi(q);
+        }
+    }
+}
+
+// CTAs and the visibilities each takes: every CTA resident at once, each with
+// an equal contiguous run.
+static void romein_split(int64_t n, int64_t resident, int64_t *blocks, int64_t *chunk)
+{
+    *chunk = (n + resident - 1) / resident;
+    if (*chunk < 8) *chunk = 8;
+    *blocks = (n + *chunk - 1) / *chunk;
+    if (*blocks < 1) *blocks = 1;
+}
+
+template <int K, int P>
+static void romein_pairs_launch(cudaStream_t s, const int4 *rec, const float2 *visf, int64_t n, const float4 *taps,
+                                float2 *grids, const int *slot_of_bin, int64_t grid_stride, int grid_side,
+                                int sm_count, int slot_cap)
+{
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, romein_pairs_kernel<K, P>, K * K / P, 0);
+    int64_t blocks, chunk;
+    romein_split(n, (int64_t)sm_count * (per_sm < 1 ? 1 : per_sm), &blocks, &chunk);
+    romein_pairs_kernel<K, P><<<(unsigned)blocks, K * K / P, 0, s>>>(rec, visf, n, taps, grids, slot_of_bin,
+                                                                     grid_stride, grid_side, chunk, slot_cap);
+}
+
 template <int K, int P>
 static void romein_launch(cudaStream_t s, const int4 *rec, const float2 *visf, int64_t n, const float2 *taps,
                           const double2 *taps64, float2 *grids, const int *slot_of_bin, int64_t grid_stride,
                           int grid_side, int sm_count, int slot_cap, int strip_lg)
 {
-    // Every CTA resident at once, each with an equal contiguous run of
-    // visibilities: occupancy, not the chunk size, decides the grid.
-    constexpr int NT = K * K / P;
-    int per_sm = 0;  // of the instantiation that runs (the register counts can differ)
-    if (strip_lg)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, romein_kernel<K, P, true>, NT, 0);
-    else if (taps64)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, romein_kernel<K, P, false, true>, NT, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, romein_kernel<K, P, false>, NT, 0);
-    if (per_sm < 1) per_sm = 1;
-    int64_t blocks = (int64_t)sm_count * per_sm;
-    int64_t chunk = (n + blocks - 1) / blocks;
-    if (chunk < 8) chunk = 8;
-    blocks = (n + chunk - 1) / chunk;
-    if (blocks < 1) blocks = 1;
-    if (strip_lg)
-        romein_kernel<K, P, true><<<(unsigned)blocks, NT, 0, s>>>(rec, visf, n, taps, nullptr, grids, slot_of_bin,
-                                                                  grid_stride, grid_side, chunk, slot_cap, strip_lg);
-    else if (taps64)
-        romein_kernel<K, P, false, true><<<(unsigned)blocks, NT, 0, s>>>(rec, visf, n, nullptr, taps64, grids,
-                                                                         slot_of_bin, grid_stride, grid_side, chunk,
-                                                                         slot_cap, 0);
-    else
-        romein_kernel<K, P, false><<<(unsigned)blocks, NT, 0, s>>>(rec, visf, n, taps, nullptr, grids, slot_of_bin,
-                                                                   grid_stride, grid_side, chunk, slot_cap, 0);
+    auto go = [&](auto kernel) {
+        int per_sm = 0;  // of the instantiation that runs (the register counts can differ)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, K * K / P, 0);
+        int64_t blocks, chunk;
+        romein_split(n, (int64_t)sm_count * (per_sm < 1 ? 1 : per_sm), &blocks, &chunk);
+        kernel<<<(unsigned)blocks, K * K / P, 0, s>>>(rec, visf, n, taps, taps64, grids, slot_of_bin, grid_stride,
+                                                      grid_side, chunk, slot_cap, strip_lg);
+    };
+    if (strip_lg) go(romein_kernel<K, P, true>);
+    else if (taps64) go(romein_kernel<K, P, false, true>);
+    else if constexpr (K < 16) go(romein_kernel<K, P, false>);  // larger supports read converted tables in pairs
 }
 
 void launch_romein(cudaStream_t s, const int4 *rec, const float2 *visf, int64_t n,
@@ -230,6 +375,10 @@ void launch_romein(cudaStream_t s, const int4 *rec, const float2 *visf, int64_t 
 #define RG_ROMEIN(K, P) \
     romein_launch<K, P>(s, rec, visf, n, taps, taps64, grids, slot_of_bin, grid_stride, grid_side, sm_count, \
                         slot_cap, strip_lg)
+#define RG_PAIRS(K, P)                                                                                     \
+    romein_pairs_launch<K, P>(s, rec, visf, n, (const float4 *)taps, grids, slot_of_bin, grid_stride, grid_side, \
+                              sm_count, slot_cap)
+    const bool pairs = !strip_lg && !taps64;  // a converted table of 16 or 32 cells, row-major
     switch (ksize) {
         case 4: RG_ROMEIN(4, 1); break;
         case 8:
@@ -238,16 +387,19 @@ void launch_romein(cudaStream_t s, const int4 *rec, const float2 *visf, int64_t 
             else RG_ROMEIN(8, 2);
             break;
         case 16:
-            if (points == 2) RG_ROMEIN(16, 2);
+            if (pairs) RG_PAIRS(16, 8);
+            else if (points == 2) RG_ROMEIN(16, 2);
             else if (points == 8) RG_ROMEIN(16, 8);
             else RG_ROMEIN(16, 4);
             break;
         case 32:
-            if (points == 8) RG_ROMEIN(32, 8);
+            if (pairs) RG_PAIRS(32, 8);
+            else if (points == 8) RG_ROMEIN(32, 8);
             else RG_ROMEIN(32, 4);
             break;
         default: break;
     }
+#undef RG_PAIRS
 #undef RG_ROMEIN
 }
 

@@ -190,18 +190,15 @@ static rg_status stage_vis(rg_context *ctx, const rg_vis *vis, DevVis *dv)
     return RG_OK;
 }
 
-// dup: the W-towers layout with each slice stored twice (launch_convert_table_dup)
-static rg_status stage_taps(rg_context *ctx, const rg_wkern *wk, float2 **taps, bool dup = false)
+// strips: for the W-towers sub-grids (launch_convert_taps)
+static rg_status stage_taps(rg_context *ctx, const rg_wkern *wk, float2 **taps, bool strips = false)
 {
     const int64_t ntaps = (int64_t)wk->plane_count * wk->oversampling * wk->oversampling * wk->size * wk->size;
     const void *src;
     RG_CHECK(stage_in(ctx, wk->data, sizeof(double2) * ntaps, "in_wkern", &src));
     void *dst;
-    RG_CHECK(scratch(ctx, dup ? "taps32_dup" : "taps32", sizeof(float2) * ntaps * (dup ? 2 : 1), &dst));
-    if (dup)
-        launch_convert_table_dup(ctx->stream, (const double2 *)src, (float2 *)dst, ntaps, wk->size * wk->size);
-    else
-        launch_convert_table(ctx->stream, (const double2 *)src, (float2 *)dst, ntaps);
+    RG_CHECK(scratch(ctx, strips ? "taps32_dup" : "taps32", sizeof(float2) * ntaps * (strips ? 2 : 1), &dst));
+    launch_convert_taps(ctx->stream, (const double2 *)src, (float2 *)dst, ntaps, wk->size, strips);
     ctx->launches++;
     *taps = (float2 *)dst;
     return check_launch("convert w-kernel table");

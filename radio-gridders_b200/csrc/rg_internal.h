@@ -201,10 +201,11 @@ rg_status visit_vis_hdf5(const char *path, double bl_min, double bl_max,
 // ---------------------------------------------------------------------------
 
 // k_image.cu
-void launch_convert_table(cudaStream_t s, const double2 *src, float2 *dst, int64_t n);
-// The W-towers gridder's copy: every K x K slice stored twice (2 K^2 taps), so
-// a thread's rows (r0 + j) mod K are read as r0 + j without wrapping.
-void launch_convert_table_dup(cudaStream_t s, const double2 *src, float2 *dst, int64_t n, int kk);
+// The FP32 kernel table in the layout launch_romein reads. Strip-major sub-grids:
+// every K x K slice twice (2 K^2 taps), so a thread's rows (r0 + j) mod K are
+// read as r0 + j without wrapping. Row-major grids: rows r and r + K/2 of a slice
+// in one entry for 16 and 32 cells, the taps as they are for 4 and 8.
+void launch_convert_taps(cudaStream_t s, const double2 *src, float2 *dst, int64_t n, int ksize, bool strips);
 void launch_make_hermitian(cudaStream_t s, double2 *grid, int n);
 void launch_fft_shift(cudaStream_t s, double2 *grid, int n);
 void launch_weight_count(cudaStream_t s, const double *u, const double *v, int64_t nvis,

@@ -139,7 +139,7 @@ extern "C" rg_status rg_grid_wprojection_noalloc(double *uvgrid, int grid_size, 
     // the array keeps the previous call's contents: clear what must start at zero
     RG_CUDA(cudaMemsetAsync(grid32, 0, sizeof(float2) * cells, st));
     RG_CUDA(cudaMemsetAsync(base + kOffMisc, 0, kMiscBytes, st));
-    launch_convert_table(st, (const double2 *)wkern->data, taps32, ntaps);
+    launch_convert_taps(st, (const double2 *)wkern->data, taps32, ntaps, K, false);
     for (int64_t off = 0; off < vis->n; off += kBatch) {
         const int64_t cnt = vis->n - off < kBatch ? vis->n - off : kBatch;
         launch_prepare_wproj(st, vis->u + off, vis->v + off, vis->w + off,

@@ -349,3 +349,68 @@ def test_wtowers_cuts_on_the_boundaries(rg, ctx, sim, oracle):
     assert rel_rms(g, ref) < TOL
     st = ctx.last_stats()
     assert st["gridded"] == int(counts.sum()) and st["gridded"] + st["dropped"] == m
+
+
+def _walk(rng, n, lim, step):
+    """Positions (cells) that stand still, step one or two cells along either
+    axis, cross K cells at once and jump, staying within +-lim."""
+    x = np.zeros((n, 2))
+    for i in range(1, n):
+        kind = rng.integers(0, 8)
+        d = np.zeros(2)
+        if kind == 7:
+            x[i] = rng.uniform(-lim, lim, 2)
+            continue
+        if kind >= 2:
+            d[rng.integers(0, 2)] = rng.choice([-2, -1, 1, 2, -step, step])
+        if kind == 6:
+            d = rng.choice([-1.0, 1.0], 2)
+        x[i] = np.where(np.abs(x[i - 1] + d) <= lim, x[i - 1] + d, x[i - 1] - d)
+    return x + rng.uniform(-0.2, 0.2, x.shape)
+
+
+# the points' moves of the sub-grid gridder: every step of a footprint's origin
+# against its wrapping, towers' edges (margin = K), every support, schedules by
+# default and tuned
+@pytest.mark.parametrize("ksize,tuned", [(4, False), (8, False), (8, True), (16, False), (16, True), (32, False),
+                                         (32, True)])
+def test_wtowers_footprint_moves(rg, sim, oracle, ksize, tuned):
+    rng = np.random.default_rng(ksize)
+    n, th, winc = 256, 0.1, 10.0
+    x = _walk(rng, 3000, n / 2 - ksize, ksize)
+    u, v = np.ascontiguousarray(x[:, 0] / th), np.ascontiguousarray(x[:, 1] / th)
+    w = np.repeat(rng.uniform(-15, 15, 300), 10)
+    vis = rng.normal(size=3000) + 1j * rng.normal(size=3000)
+    wk = sim.generate_wkernel(th, np.arange(-5.0, 6.0), ksize, 4)
+    ctx = rg.Context(0)
+    ctx.set_autotune(tuned)
+    g = np.zeros((n, n), np.complex128)
+    ctx.grid_wtowers(g, n, th, V(rg, u, v, w, vis), wk, 128, max(ksize, 16), winc)
+    ref = oracle.grid_wtowers(n, th, u, v, w, vis, wk, 128, max(ksize, 16), winc)
+    assert rel_rms(g, ref) < TOL
+    ctx.close()
+
+
+@pytest.mark.parametrize("ksize", [4, 8, 16, 32])
+def test_wprojection_footprint_moves(rg, ctx, sim, ksize):
+    """The converted-table gridder's moves and grid edges against an FP64 scatter
+    that drops each tap off the grid."""
+    rng = np.random.default_rng(100 + ksize)
+    n, th, ov = 90, 0.1, 2
+    x = _walk(rng, 2000, n / 2, ksize)
+    u, v = np.ascontiguousarray(x[:, 0] / th), np.ascontiguousarray(x[:, 1] / th)
+    w = rng.uniform(-9, 9, 2000)
+    vis = rng.normal(size=2000) + 1j * rng.normal(size=2000)
+    wk = sim.generate_wkernel(th, np.arange(-1.0, 2.0) * 10.0, ksize, ov)
+    g = np.zeros((n, n), np.complex128)
+    ctx.grid_wprojection(g, n, th, V(rg, u, v, w, vis), wk)
+    pad = 2 * ksize
+    ref = np.zeros((n + 2 * pad, n + 2 * pad), np.complex128)
+    cx, cy = np.floor(th * u + 0.5 / ov).astype(int), np.floor(th * v + 0.5 / ov).astype(int)
+    fx = np.floor((th * u - cx) * ov + 0.5).astype(int)
+    fy = np.floor((th * v - cy) * ov + 0.5).astype(int)
+    pl = np.floor((w - wk.w_min) / wk.w_step + 0.5).astype(int)
+    for i in range(2000):
+        r0, c0 = cy[i] + n // 2 - ksize // 2 + pad, cx[i] + n // 2 - ksize // 2 + pad
+        ref[r0:r0 + ksize, c0:c0 + ksize] += vis[i] * np.conj(wk.data[pl[i], fy[i], fx[i]])
+    assert rel_rms(g, ref[pad:-pad, pad:-pad]) < TOL
