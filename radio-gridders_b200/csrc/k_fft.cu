@@ -320,33 +320,38 @@ __global__ void __launch_bounds__(kSparseColThreads) sparse_cols_kernel(
 // ---------------------------------------------------------------------------
 // Row stage, in two kernels so uneven towers balance.
 //
-// tower_rows_kernel: CTA = (floor group, R rows: four mirror pairs (y, N - y)
-// when R = 8, so each Fresnel factor serves two rows; else a strip).  For each floor of
-// the group: backward row transform of the column-transformed sub-grid (only
-// the slot's marked strips are read, then zeroed), times exp(-2 pi i wp
-// ph(l, m)) with ph = winc (1 - sqrt(1 - l^2 - m^2)) — the reference's
-// wtransfer^(-wp), grid.c:304-319 and :473-496, which also covers the w = 0
-// transfer — accumulated in registers; the strip sum goes to the group's
-// partial buffer.  The phase -wp * ph is formed modulo one turn as an integer
-// product with the 32-bit fixed-point table (fresnel_table_kernel), converted
-// to FP32 (24 significant bits) for sin/cos.
+// tower_rows_kernel: CTA = (floor group, 128/N1 rows), four warps that never wait
+// for one another: a warp owns 32/N1 rows, whose 32 step-1 transforms are one a
+// lane, whose exchange stays in the warp's part of shared memory and whose
+// step-2 transforms (a lane is one k2 of each row) its lanes accumulate. For each
+// floor of the group: backward row transform of the column-transformed sub-grid
+// (only the slot's marked strips are read, then zeroed), times
+// exp(-2 pi i wp ph(l, m)) with ph = winc (1 - sqrt(1 - l^2 - m^2)) — the
+// reference's wtransfer^(-wp), grid.c:304-319 and :473-496, which also covers the
+// w = 0 transfer — accumulated in registers; the sums go to the group's partial
+// buffer. Rows come in mirror pairs (y, N - y) so each Fresnel factor serves two.
+// The phase -wp * ph is formed modulo one turn as an integer product with the
+// 32-bit fixed-point table (fresnel_table_kernel), converted to FP32 (24
+// significant bits) for sin/cos. Bound by instruction issue and by the latency
+// of the strip loads. N = 512, 998 sub-grids: 536 -> 489 us; N = 128, 22,464
+// visibilities: 92 -> 28 us (there one warp of four had done all of step 1).
 //
 // tower_rows_finish_kernel: CTA = (tower, strip of R rows).  Sums the tower's
-// group partials in group order (deterministic) and applies the forward row
-// transform into the tower's sub-image (the row half of grid.c:499).
+// group partials in group order (deterministic) and applies the forward row transform into the tower's sub-image (the
+// row half of grid.c:499).
 // ---------------------------------------------------------------------------
 constexpr int kRowThreads = 128;
 template <int N1>
 struct RowGeom {
     static constexpr int N = N1 * 32;
-    static constexpr int R = N1 >= 32 ? 4 : 8;  // rows per CTA
+    static constexpr int R = kRowThreads / N1;  // rows per CTA: one step-1 item a thread
+    static constexpr int PER = R / 4;           // rows per warp: step-2 items a lane
+    static constexpr bool MIRROR = PER >= 2;    // a warp's rows are PER/2 mirror pairs
+    static constexpr int PROWS = MIRROR ? R / 2 : R;  // rows of distinct phases
     static constexpr int LB = ilog2c(N1);
     static constexpr int STRIPS = N / kStripCols;
     static constexpr int WORDS = (STRIPS + 31) / 32;
-    static constexpr int ITEMS1 = R * N1;  // step-1 items (n1, row)
-    static constexpr int ITEMS2 = R * 32;  // step-2 items (k2, row)
-    static constexpr int PER = (ITEMS2 + kRowThreads - 1) / kRowThreads;
-    static constexpr int T_ELEMS = R * N1 * kPad;
+    static constexpr int T_ELEMS = kRowThreads * kPad;
 };
 
 int tower_row_strips(int subgrid) { return subgrid / (subgrid >= 1024 ? 4 : 8); }
@@ -387,80 +392,79 @@ __device__ __forceinline__ unsigned element_bits(unsigned long long lo, unsigned
 
 // a = *p when on, else a is left as it is.  A predicated load: the register is
 // written only by the load, so no select waits on the load's result and all of
-// a thread's loads stay in flight together.  The memory clobber keeps later
-// stores (the clearing) after it.
-__device__ __forceinline__ void ld_if(float2 &a, const float2 *p, bool on)
+// a thread's loads stay in flight together.
+__device__ __forceinline__ void ld_if(unsigned long long &a, const float2 *p, bool on)
 {
     asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q ld.global.v2.f32 {%0, %1}, [%2];\n\t}"
-        : "+f"(a.x), "+f"(a.y)
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.b64 %0, [%1];\n\t}"
+        : "+l"(a)
         : "l"(p), "r"((unsigned)on)
         : "memory");
 }
 
 template <int N1>
-__global__ void __launch_bounds__(kRowThreads) tower_rows_kernel(
+__global__ void __launch_bounds__(kRowThreads, 3) tower_rows_kernel(
     float2 *__restrict__ slots, const unsigned *__restrict__ masks, const int *__restrict__ bin_of_slot,
     const int *__restrict__ group_begin, const int *__restrict__ group_end, const int *__restrict__ range,
     const int *__restrict__ counts, int slot_cap, const uint32_t *__restrict__ phq, float2 *__restrict__ partial,
     const float2 *__restrict__ tw)
 {
     using G = RowGeom<N1>;
-    constexpr int N = G::N, R = G::R;
+    constexpr int N = G::N, R = G::R, PER = G::PER;
     extern __shared__ float2 smem[];
-    float2 *T = smem;                                // [R][N1][kPad]
-    float2 *W = smem + G::T_ELEMS;                   // [N]
-    uint32_t *P = reinterpret_cast<uint32_t *>(W + N);  // [R][N] Fresnel phase of the strip (turns, 2^-32)
-    __shared__ unsigned smask[G::WORDS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2 *T = smem + warp * 32 * kPad;                // [PER][N1][kPad], this warp's
+    float2 *W = smem + G::T_ELEMS;                      // [N]
+    uint32_t *P = reinterpret_cast<uint32_t *>(W + N);  // [PROWS][N] Fresnel phases (turns, 2^-32)
     const int rstrips = N / R;
     const int group = blockIdx.x / rstrips, blk = blockIdx.x % rstrips;
     if (group >= counts[1]) return;  // groups live on the device; grid sized for capacity
-    // MIRROR: the CTA's rows are four mirror pairs (y, N - y) — pair p is
-    // (p, N - p), pair 0 is (0, N/2) — local rows 0-3 the first rows and 4-7
-    // their mirrors.  ph(l, m) depends on m^2 only and the table's rows y and
-    // N - y hold the same values, so a thread's two step-2 items (the same
-    // column, rows r and r + 4) share each Fresnel factor, except in pair 0.
-    constexpr bool MIRROR = R == 8 && G::PER == 2 && G::ITEMS2 == 2 * kRowThreads;
-    auto row_of = [&](int r) -> int {
-        if constexpr (!MIRROR) {
-            return blk * R + r;
-        } else {
-            const int p = 4 * blk + (r & 3);
-            return r < 4 ? p : (p == 0 ? N / 2 : N - p);
-        }
+    // Row i of the warp. Mirror pair p is rows p and N - p, pair 0 rows 0 and N/2:
+    // ph(l, m) depends on m^2 only and the table's rows y and N - y hold the same
+    // values, so a pair shares each Fresnel factor, except pair 0.
+    const int first = (blk * 4 + warp) * (G::MIRROR ? PER / 2 : PER);  // the warp's first pair or row
+    auto row_of = [&](int i) -> int {
+        if constexpr (!G::MIRROR) return first + i;
+        const int p = first + (i >> 1);
+        return i & 1 ? (p == 0 ? N / 2 : N - p) : p;
     };
     const int wp_min = range[0], nfloor = range[1];
     const int begin = group_begin[group];
     const int end = group_end[group] < slot_cap ? group_end[group] : slot_cap;
     load_twiddles<N1>(W, tw);
-    for (int e = threadIdx.x; e < R * N; e += blockDim.x) P[e] = phq[(int64_t)row_of(e / N) * N + e % N];
+    for (int e = threadIdx.x; e < G::PROWS * N; e += blockDim.x) P[e] = phq[(int64_t)blk * G::PROWS * N + e];
+    P += warp * (G::PROWS / 4) * N;
+    __syncthreads();  // the only wait between the warps
 
-    float2 acc[G::PER][N1];
+    float2 acc[PER][N1];
 #pragma unroll
-    for (int q = 0; q < G::PER; q++)
+    for (int q = 0; q < PER; q++)
 #pragma unroll
         for (int j = 0; j < N1; j++) acc[q][j] = make_float2(0.f, 0.f);
 
+    // the lane's step-1 item: columns n1 + n2 N1 of row i
+    const int n1 = lane % N1, i1 = lane / N1;
+    const int64_t row_at = (int64_t)row_of(i1) * kStripCols;
     // the next floor's strip mask is loaded a floor ahead, so only the strip
     // loads wait on memory at the top of a floor
-    unsigned mnext = (threadIdx.x < G::WORDS && begin < end) ? masks[(int64_t)begin * G::WORDS + threadIdx.x] : 0u;
+    unsigned mnext[G::WORDS];
+#pragma unroll
+    for (int k = 0; k < G::WORDS; k++) mnext[k] = begin < end ? __ldg(masks + (int64_t)begin * G::WORDS + k) : 0u;
     for (int slot = begin; slot < end; slot++) {
         const uint32_t mwp = (uint32_t)(-(wp_min + bin_of_slot[slot] % nfloor));  // two's complement
-        if (threadIdx.x < G::WORDS) {
-            smask[threadIdx.x] = mnext;
-            if (slot + 1 < end) mnext = masks[(int64_t)(slot + 1) * G::WORDS + threadIdx.x];
-        }
-        __syncthreads();  // masks visible; the previous floor's step 2 is done with T
         // the slot's strip mask in two 64-bit registers (at most 128 strips)
-        const unsigned long long m_lo = smask[0] | (G::WORDS > 1 ? (unsigned long long)smask[1] << 32 : 0ull);
+        const unsigned long long m_lo = mnext[0] | (G::WORDS > 1 ? (unsigned long long)mnext[G::WORDS > 1] << 32 : 0ull);
         const unsigned long long m_hi =
-            G::WORDS > 2 ? (smask[2] | (G::WORDS > 3 ? (unsigned long long)smask[3] << 32 : 0ull)) : 0ull;
-        for (int it = threadIdx.x; it < G::ITEMS1; it += blockDim.x) {
-            const int n1 = it % N1, r = it / N1;
-            // strip-major sub-grid: column col of row (row0 + r) at (col/8)*8N + row*8 + col%8;
-            // for N1 >= 8 element n2 lies n2 * (N1/8) strips after the thread's first,
-            // a compile-time offset from one per-thread base
-            float2 *row_base = slots + (int64_t)slot * N * N + row_of(r) * kStripCols;
+            G::WORDS > 2 ? (mnext[G::WORDS > 2 ? 2 : 0] | (unsigned long long)mnext[G::WORDS > 2 ? 3 : 0] << 32) : 0ull;
+        if (slot + 1 < end) {
+#pragma unroll
+            for (int k = 0; k < G::WORDS; k++) mnext[k] = __ldg(masks + (int64_t)(slot + 1) * G::WORDS + k);
+        }
+        {
+            // strip-major sub-grid: column col of a row at (col/8)*8N + row*8 + col%8;
+            // for N1 >= 8 element n2 lies n2 * (N1/8) strips after the lane's first,
+            // a compile-time offset from one base
+            float2 *row_base = slots + (int64_t)slot * N * N + row_at;
             float2 *src = row_base + (n1 / kStripCols) * (kStripCols * N) + n1 % kStripCols;
             auto elem = [&](int n2) -> float2 * {
                 if constexpr (N1 >= kStripCols) {
@@ -471,24 +475,25 @@ __global__ void __launch_bounds__(kRowThreads) tower_rows_kernel(
                 }
             };
             const unsigned on = element_bits<N1>(m_lo, m_hi, n1);
-            float2 a[32];
-            // all 32 loads issue before any clearing store
+            unsigned long long raw[32];
 #pragma unroll
             for (int n2 = 0; n2 < 32; n2++) {
-                a[n2] = make_float2(0.f, 0.f);
-                ld_if(a[n2], elem(n2), (on >> n2) & 1u);
+                raw[n2] = 0;
+                ld_if(raw[n2], elem(n2), (on >> n2) & 1u);
             }
+            float2 a[32];
 #pragma unroll
             for (int n2 = 0; n2 < 32; n2++)
-                if ((on >> n2) & 1u) *elem(n2) = make_float2(0.f, 0.f);  // leave the sub-grid zeroed
+                a[n2] = make_float2(__uint_as_float((unsigned)raw[n2]), __uint_as_float((unsigned)(raw[n2] >> 32)));
             reg_fft<32, +1>(a);
+            __syncwarp();  // the previous floor's step 2 has read T
 #pragma unroll
             for (int j = 0; j < 32; j++) {
                 const int k2 = bitrevc(j, 5);
-                T[(r * N1 + n1) * kPad + k2] = cmulf(a[j], twiddle<+1>(W, k2 * N1 + n1));
+                T[(i1 * N1 + n1) * kPad + k2] = cmulf(a[j], twiddle<+1>(W, k2 * N1 + n1));
             }
         }
-        __syncthreads();
+        __syncwarp();
         // -wp ph modulo one turn as a signed 32-bit fraction of a turn, rounded
         // to 24 significant bits by the conversion (at most 64 units of 2^-32,
         // 2^-26 turns, off); acc += b * (cs + i sn) as two packed-pair fused
@@ -501,68 +506,93 @@ __global__ void __launch_bounds__(kRowThreads) tower_rows_kernel(
             a = __ffma2_rn(make_float2(v.x, v.x), make_float2(cs, sn), a);
             a = __ffma2_rn(make_float2(v.y, v.y), make_float2(-sn, cs), a);
         };
-        if constexpr (MIRROR) {
-            const int k2 = threadIdx.x % 32, r = threadIdx.x / 32;  // items (k2, r) and (k2, r + 4)
-            float2 b0[N1], b1[N1];
+        if constexpr (G::MIRROR) {
 #pragma unroll
-            for (int n1 = 0; n1 < N1; n1++) {
-                b0[n1] = T[(r * N1 + n1) * kPad + k2];
-                b1[n1] = T[((r + 4) * N1 + n1) * kPad + k2];
-            }
-            reg_fft<N1, +1>(b0);
-            reg_fft<N1, +1>(b1);
-            if (blk != 0 || r != 0) {  // a mirror pair: one factor for both rows
+            for (int q = 0; q < PER; q += 2) {  // a pair: rows q and q + 1 of the warp, k2 = lane
+                float2 b0[N1], b1[N1];
 #pragma unroll
-                for (int j = 0; j < N1; j++) {
-                    const int col = k2 + 32 * bitrevc(j, G::LB);
-                    float sn, cs;
-                    fresnel(P[r * N + col], sn, cs);
-                    accumulate(acc[0][j], b0[j], sn, cs);
-                    accumulate(acc[1][j], b1[j], sn, cs);
+                for (int m = 0; m < N1; m++) {
+                    b0[m] = T[(q * N1 + m) * kPad + lane];
+                    b1[m] = T[((q + 1) * N1 + m) * kPad + lane];
                 }
-            } else {  // pair 0: rows 0 and N/2
+                reg_fft<N1, +1>(b0);
+                reg_fft<N1, +1>(b1);
+                const uint32_t *ph = P + (q / 2) * N + lane;
+                if (first + q / 2 != 0) {  // one factor for both rows
 #pragma unroll
-                for (int j = 0; j < N1; j++) {
-                    const int col = k2 + 32 * bitrevc(j, G::LB);
-                    float sn, cs;
-                    fresnel(P[r * N + col], sn, cs);
-                    accumulate(acc[0][j], b0[j], sn, cs);
-                    fresnel(P[(r + 4) * N + col], sn, cs);
-                    accumulate(acc[1][j], b1[j], sn, cs);
+                    for (int j = 0; j < N1; j++) {
+                        float sn, cs;
+                        fresnel(ph[32 * bitrevc(j, G::LB)], sn, cs);
+                        accumulate(acc[q][j], b0[j], sn, cs);
+                        accumulate(acc[q + 1][j], b1[j], sn, cs);
+                    }
+                } else {  // pair 0: rows 0 and N/2
+#pragma unroll
+                    for (int j = 0; j < N1; j++) {
+                        float sn, cs;
+                        fresnel(ph[32 * bitrevc(j, G::LB)], sn, cs);
+                        accumulate(acc[q][j], b0[j], sn, cs);
+                        fresnel(__ldg(phq + (int64_t)(N / 2) * N + lane + 32 * bitrevc(j, G::LB)), sn, cs);
+                        accumulate(acc[q + 1][j], b1[j], sn, cs);
+                    }
                 }
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < G::PER; q++) {
-                const int it = threadIdx.x + q * kRowThreads;
-                if (it < G::ITEMS2) {
-                    const int k2 = it % 32, r = it / 32;
-                    float2 b[N1];
+            for (int q = 0; q < PER; q++) {
+                float2 b[N1];
 #pragma unroll
-                    for (int n1 = 0; n1 < N1; n1++) b[n1] = T[(r * N1 + n1) * kPad + k2];
-                    reg_fft<N1, +1>(b);
+                for (int m = 0; m < N1; m++) b[m] = T[(q * N1 + m) * kPad + lane];
+                reg_fft<N1, +1>(b);
 #pragma unroll
-                    for (int j = 0; j < N1; j++) {
-                        float sn, cs;
-                        fresnel(P[r * N + k2 + 32 * bitrevc(j, G::LB)], sn, cs);
-                        accumulate(acc[q][j], b[j], sn, cs);
-                    }
+                for (int j = 0; j < N1; j++) {
+                    float sn, cs;
+                    fresnel(P[q * N + lane + 32 * bitrevc(j, G::LB)], sn, cs);
+                    accumulate(acc[q][j], b[j], sn, cs);
+                }
+            }
+        }
+        // Leave the marked strips zeroed, 16 bytes a lane, eight (strip, row) pieces
+        // a store: at the end of the floor, behind a barrier. Beside the loads the
+        // compiler pairs each load with its clear and waits for one after the
+        // other (2553 us in place of 536 for the whole stage).
+        __syncwarp();
+        {
+            constexpr int ROWS = PER < 8 ? PER : 8;  // rows a store covers, the lanes' pieces / ROWS its strips
+            const int piece = lane >> 2, s0 = piece / ROWS;
+            const unsigned long long c_lo = m_lo >> s0, c_hi = m_hi >> s0;
+#pragma unroll
+            for (int h = 0; h < PER; h += ROWS) {
+                float2 *at = slots + (int64_t)slot * N * N + (int64_t)s0 * (kStripCols * N) +
+                             row_of(h + piece % ROWS) * kStripCols + 2 * (lane & 3);
+#pragma unroll
+                for (int st = 0; st < G::STRIPS; st += 8 / ROWS) {
+                    const unsigned half = (unsigned)((st & 64 ? c_hi : c_lo) >> (st & 32));
+                    if (half & (1u << (st & 31)))
+                        *reinterpret_cast<float4 *>(at + st * (kStripCols * N)) = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }
         }
     }
     float2 *out = partial + (int64_t)group * N * N;
 #pragma unroll
-    for (int q = 0; q < G::PER; q++) {
-        const int it = threadIdx.x + q * kRowThreads;
-        if (it < G::ITEMS2) {
-            const int k2 = it % 32, r = it / 32;
-            float2 *o = out + (int64_t)row_of(r) * N + k2;
+    for (int q = 0; q < PER; q++) {
+        float2 *o = out + (int64_t)row_of(q) * N + lane;
 #pragma unroll
-            for (int j = 0; j < N1; j++) o[32 * bitrevc(j, G::LB)] = acc[q][j];
-        }
+        for (int j = 0; j < N1; j++) o[32 * bitrevc(j, G::LB)] = acc[q][j];
     }
 }
+
+// The finish kernel's strips: 8 rows (4 at N = 1024).
+template <int N1>
+struct FinishGeom {
+    static constexpr int N = N1 * 32;
+    static constexpr int R = N1 >= 32 ? 4 : 8;
+    static constexpr int LB = ilog2c(N1);
+    static constexpr bool SPREAD = R * N1 < kRowThreads;
+    static constexpr int PER = R * N / kRowThreads;  // elements a thread sums when spread
+    static constexpr int T_ELEMS = R * N1 * kPad;
+};
 
 template <int N1>
 __global__ void __launch_bounds__(kRowThreads) tower_rows_finish_kernel(
@@ -570,11 +600,12 @@ __global__ void __launch_bounds__(kRowThreads) tower_rows_finish_kernel(
     const int *__restrict__ tower_group_count, int group_cap, float2 *__restrict__ subimg,
     const float2 *__restrict__ tw)
 {
-    using G = RowGeom<N1>;
+    using G = FinishGeom<N1>;
     constexpr int N = G::N, R = G::R;
     extern __shared__ float2 smem[];
     float2 *T = smem;
     float2 *W = smem + G::T_ELEMS;
+    float2 *X = W + N;  // [R][N]: the strip's sums, when spread
     const int rstrips = N / R;
     const int tower = blockIdx.x / rstrips, row0 = (blockIdx.x % rstrips) * R;
     const int gfirst = tower_group_first[tower];
@@ -582,17 +613,35 @@ __global__ void __launch_bounds__(kRowThreads) tower_rows_finish_kernel(
     if (gfirst + gcount > group_cap) gcount = group_cap - gfirst;  // capacity overflow: rerun
     if (gcount <= 0) return;
     load_twiddles<N1>(W, tw);
+    // Summed by the step-1 items themselves where they are as many as the threads,
+    // else by all threads through shared memory (N = 128: 28 -> 9 us for 25 towers
+    // of 19 groups; at N = 512 the way through shared memory costs 20 -> 34 us)
+    constexpr bool SPREAD = G::SPREAD;
+    const float2 *strip = partial + ((int64_t)gfirst * N + row0) * N;
+    if constexpr (SPREAD) {
+        float2 a[G::PER];
+#pragma unroll
+        for (int k = 0; k < G::PER; k++) a[k] = make_float2(0.f, 0.f);
+        const float2 *src = strip + threadIdx.x;
+        for (int g = 0; g < gcount; g++, src += (int64_t)N * N) {
+#pragma unroll
+            for (int k = 0; k < G::PER; k++) a[k] = caddf(a[k], src[k * kRowThreads]);
+        }
+#pragma unroll
+        for (int k = 0; k < G::PER; k++) X[k * kRowThreads + threadIdx.x] = a[k];
+    }
     __syncthreads();
-    for (int it = threadIdx.x; it < G::ITEMS1; it += blockDim.x) {
+    for (int it = threadIdx.x; it < R * N1; it += blockDim.x) {
         const int n1 = it % N1, r = it / N1;
         float2 a[32];
 #pragma unroll
-        for (int n2 = 0; n2 < 32; n2++) a[n2] = make_float2(0.f, 0.f);
-        for (int g = 0; g < gcount; g++) {
-            const float2 *src = partial + ((int64_t)(gfirst + g) * N + row0 + r) * N + n1;
+        for (int n2 = 0; n2 < 32; n2++) a[n2] = SPREAD ? X[r * N + n1 + n2 * N1] : make_float2(0.f, 0.f);
+        if constexpr (!SPREAD)
+            for (int g = 0; g < gcount; g++) {
+                const float2 *src = strip + ((int64_t)g * N + r) * N + n1;
 #pragma unroll
-            for (int n2 = 0; n2 < 32; n2++) a[n2] = caddf(a[n2], src[n2 * N1]);
-        }
+                for (int n2 = 0; n2 < 32; n2++) a[n2] = caddf(a[n2], src[n2 * N1]);
+            }
         reg_fft<32, -1>(a);
 #pragma unroll
         for (int j = 0; j < 32; j++) {
@@ -602,7 +651,7 @@ __global__ void __launch_bounds__(kRowThreads) tower_rows_finish_kernel(
     }
     __syncthreads();
     float2 *out = subimg + ((int64_t)tower * N + row0) * N;
-    for (int it = threadIdx.x; it < G::ITEMS2; it += blockDim.x) {
+    for (int it = threadIdx.x; it < R * 32; it += blockDim.x) {
         const int k2 = it % 32, r = it / 32;
         float2 b[N1];
 #pragma unroll
@@ -625,10 +674,13 @@ static size_t sparse_cols_smem() { return sizeof(float2) * (StripGeom<N1>::T_ELE
 template <int N1>
 static size_t tower_rows_smem()
 {
-    return sizeof(float2) * (RowGeom<N1>::T_ELEMS + N1 * 32) + sizeof(uint32_t) * RowGeom<N1>::R * N1 * 32;
+    return sizeof(float2) * (RowGeom<N1>::T_ELEMS + N1 * 32) + sizeof(uint32_t) * RowGeom<N1>::PROWS * N1 * 32;
 }
 template <int N1>
-static size_t tower_finish_smem() { return sizeof(float2) * (RowGeom<N1>::T_ELEMS + N1 * 32); }
+static size_t tower_finish_smem()
+{
+    return sizeof(float2) * (FinishGeom<N1>::T_ELEMS + N1 * 32 + (FinishGeom<N1>::SPREAD ? FinishGeom<N1>::R * N1 * 32 : 0));
+}
 
 template <int N1>
 static void rows_impl(cudaStream_t s, float2 *data, int64_t rows, int sign, const float2 *tw,
@@ -691,7 +743,7 @@ static void tower_finish_impl(cudaStream_t s, int group_cap, const int *tower_gr
                               const int *tower_group_count, int ntowers, const float2 *partial, float2 *subimg,
                               const float2 *tw)
 {
-    const int rstrips = RowGeom<N1>::N / RowGeom<N1>::R;
+    const int rstrips = FinishGeom<N1>::N / FinishGeom<N1>::R;
     const size_t sm2 = tower_finish_smem<N1>();
     cudaFuncSetAttribute(tower_rows_finish_kernel<N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
     tower_rows_finish_kernel<N1><<<(unsigned)ntowers * rstrips, kRowThreads, sm2, s>>>(
