@@ -66,54 +66,83 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Element (i, k) of A and (k, n) of B, with optional transposition of the
-// stored row-major arrays.
+// Four (two) 8 x 8 tiles of 16-bit elements from shared memory, each lane giving
+// the address of one row of one tile; T: transposed.
 template <bool T>
-__device__ __forceinline__ bf16 at(const bf16 *M, int ld, int r, int c)
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const bf16 *row)
 {
-    return T ? M[c * ld + r] : M[r * ld + c];
+    const unsigned a = (unsigned)__cvta_generic_to_shared(row);
+    if (T)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }
 
-// One warp accumulates the WM x WN tile at (m0, n0) of C = A(MxK) * B(KxN).
+// One warp accumulates the WM x WN tile at (m0, n0) of C = A(MxK) * B(KxN), A in
+// shared memory as [m][k] or, TA, [k][m]. B as [n][k] in global memory (TB: the
+// weights, read as packed pairs) or as [k][n] in shared memory.
 template <int WM, int WN, bool TA, bool TB>
 __device__ __forceinline__ void warp_gemm(const bf16 *A, int lda, const bf16 *B, int ldb, int K,
                                           int m0, int n0, float (&acc)[WM / 16][WN / 8][4])
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int lr = lane & 7, lt = lane >> 3;  // ldmatrix: this lane's row and tile
+#pragma unroll 2
     for (int k0 = 0; k0 < K; k0 += 16) {
-        uint32_t a[WM / 16][4];
+        uint32_t a[WM / 16][4], b[WN / 8][2];
 #pragma unroll
         for (int mi = 0; mi < WM / 16; mi++) {
-            const int r = m0 + mi * 16 + g;
-            const int c = k0 + 2 * t;
-            if (!TA) {
-                a[mi][0] = *reinterpret_cast<const uint32_t *>(A + r * lda + c);
-                a[mi][1] = *reinterpret_cast<const uint32_t *>(A + (r + 8) * lda + c);
-                a[mi][2] = *reinterpret_cast<const uint32_t *>(A + r * lda + c + 8);
-                a[mi][3] = *reinterpret_cast<const uint32_t *>(A + (r + 8) * lda + c + 8);
-            } else {
-                a[mi][0] = pack_bf16(at<true>(A, lda, r, c), at<true>(A, lda, r, c + 1));
-                a[mi][1] = pack_bf16(at<true>(A, lda, r + 8, c), at<true>(A, lda, r + 8, c + 1));
-                a[mi][2] = pack_bf16(at<true>(A, lda, r, c + 8), at<true>(A, lda, r, c + 9));
-                a[mi][3] = pack_bf16(at<true>(A, lda, r + 8, c + 8), at<true>(A, lda, r + 8, c + 9));
-            }
+            // tiles: (m, k), (m + 8, k), (m, k + 8), (m + 8, k + 8)
+            const int m = m0 + mi * 16 + (lt & 1) * 8, k = k0 + (lt >> 1) * 8;
+            ldmatrix4<TA>(a[mi], TA ? A + (k + lr) * lda + m : A + (m + lr) * lda + k);
         }
 #pragma unroll
-        for (int ni = 0; ni < WN / 8; ni++) {
-            const int n = n0 + ni * 8 + g;
-            const int k = k0 + 2 * t;
-            uint32_t b0, b1;
+        for (int ni = 0; ni < WN / 8; ni += 2) {
+            const int n = n0 + ni * 8;
             if (TB) {
-                b0 = *reinterpret_cast<const uint32_t *>(B + n * ldb + k);
-                b1 = *reinterpret_cast<const uint32_t *>(B + n * ldb + k + 8);
-            } else {
-                b0 = pack_bf16(at<false>(B, ldb, k, n), at<false>(B, ldb, k + 1, n));
-                b1 = pack_bf16(at<false>(B, ldb, k + 8, n), at<false>(B, ldb, k + 9, n));
-            }
 #pragma unroll
-            for (int mi = 0; mi < WM / 16; mi++) mma_bf16(acc[mi][ni], a[mi][0], a[mi][1], a[mi][2], a[mi][3], b0, b1);
+                for (int h = 0; h < 2; h++) {
+                    const bf16 *row = B + (n + 8 * h + g) * ldb + k0 + 2 * t;
+                    b[ni + h][0] = __ldg(reinterpret_cast<const uint32_t *>(row));
+                    b[ni + h][1] = __ldg(reinterpret_cast<const uint32_t *>(row + 8));
+                }
+            } else {
+                // tiles: (k, n), (k + 8, n), (k, n + 8), (k + 8, n + 8), transposed
+                uint32_t r[4];
+                ldmatrix4<true>(r, B + (k0 + (lt & 1) * 8 + lr) * ldb + n + (lt >> 1) * 8);
+                b[ni][0] = r[0];
+                b[ni][1] = r[1];
+                b[ni + 1][0] = r[2];
+                b[ni + 1][1] = r[3];
+            }
         }
+#pragma unroll
+        for (int ni = 0; ni < WN / 8; ni++)
+#pragma unroll
+            for (int mi = 0; mi < WM / 16; mi++)
+                mma_bf16(acc[mi][ni], a[mi][0], a[mi][1], a[mi][2], a[mi][3], b[ni][0], b[ni][1]);
     }
+}
+
+// acc added to the row-major [rows][MH] gradient at (m0, n0): a lane's two
+// neighbouring columns by one atomic. Rows from `rows` on are left out.
+template <int WM, int WN>
+__device__ __forceinline__ void add_weight_grad(const float (&acc)[WM / 16][WN / 8][4], float *grad, int m0, int n0, int rows)
+{
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int mi = 0; mi < WM / 16; mi++)
+#pragma unroll
+        for (int ni = 0; ni < WN / 8; ni++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = m0 + mi * 16 + g + 8 * h;
+                if (r < rows)
+                    atomicAdd(reinterpret_cast<float2 *>(grad + r * MH + n0 + ni * 8 + 2 * t),
+                              make_float2(acc[mi][ni][2 * h], acc[mi][ni][2 * h + 1]));
+            }
 }
 
 template <int WM, int WN>
@@ -231,156 +260,163 @@ __device__ __forceinline__ void hidden_epilogue(const float (&acc)[WM / 16][WN /
 // training
 // ---------------------------------------------------------------------------
 constexpr int TT = 64;  // samples per CTA
+constexpr int kTrainThreads = 512;
 
 struct TrainSmem {
     bf16 F[TT * LDF];
     bf16 H[3][TT * LDH];
     float Z[3][TT * LDZ];
+    float W4[MH * 2];
     float Y[TT * 2];
+    float loss[kTrainThreads / 32];
 };
 
-// in: [5][n] float (w, du, dv, tx, ty); target: [n] float2 (unscaled taps)
-__global__ void __launch_bounds__(256) mlp_grad_kernel(const float *__restrict__ P, const bf16 *__restrict__ PB,
-                                                       const float *__restrict__ in, const float2 *__restrict__ target,
-                                                       int n, int ksize, float inv_wmax, float inv_scale,
-                                                       float *__restrict__ grad, float *__restrict__ loss)
+// in: [5][n] float (w, du, dv, tx, ty); target: [n] float2 (unscaled taps).
+// One CTA of 16 warps an SM (shared memory holds the tile's activations and FP32
+// pre-activations), so each phase's latency shows: every phase is spread over all
+// threads, operands come by ldmatrix, and each CTA adds its loss once and its
+// weight gradients two columns an atomic. 16,384 samples:
+// 127 -> 92 us.
+__global__ void __launch_bounds__(kTrainThreads) mlp_grad_kernel(
+    const float *__restrict__ P, const bf16 *__restrict__ PB, const float *__restrict__ in,
+    const float2 *__restrict__ target, int n, int ksize, float inv_wmax, float inv_scale, float *__restrict__ grad,
+    float *__restrict__ loss)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem &S = *reinterpret_cast<TrainSmem *>(smem_raw);
     const int row0 = blockIdx.x * TT;
-    const int warp = threadIdx.x >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const float inv_n = 1.f / (float)n;
 
-    if (threadIdx.x < TT) {
-        const int i = row0 + threadIdx.x;
-        if (i < n) {
-            tap_features(in[i], in[n + i], in[2 * n + i], in[3 * n + i], in[4 * n + i], ksize, inv_wmax,
-                         S.F + threadIdx.x * LDF);
-        } else {
-            for (int k = 0; k < MFIN; k++) S.F[threadIdx.x * LDF + k] = __float2bfloat16(0.f);
+    {  // features: eight threads a sample, one Fourier pair each (tap_features)
+        const int r = tid >> 3, k = (tid & 3) + 1, axis = (tid >> 2) & 1, i = row0 + r;
+        bf16 *f = S.F + r * LDF;
+        const bool on = i < n;
+        const float half = 0.5f * (float)ksize, inv = 1.f / (half + 1.f);
+        const float d = on ? in[(axis ? 2 : 1) * (int64_t)n + i] : 0.f, tap = on ? in[(axis ? 4 : 3) * (int64_t)n + i] : 0.f;
+        const float p = tap - half - d;
+        float sn, cs;
+        sincospif((float)k * p * inv, &sn, &cs);
+        f[(axis ? 13 : 5) + 2 * (k - 1)] = __float2bfloat16(on ? cs : 0.f);
+        f[(axis ? 14 : 6) + 2 * (k - 1)] = __float2bfloat16(on ? sn : 0.f);
+        if (k == 1) {
+            f[axis ? 2 : 1] = __float2bfloat16(on ? 2.f * d - 1.f : 0.f);
+            f[axis ? 4 : 3] = __float2bfloat16(on ? p / half : 0.f);
         }
+        if ((tid & 7) == 1) f[0] = __float2bfloat16(on ? in[i] * inv_wmax : 0.f);
+        for (int c = MNFEAT + (tid & 7); c < MFIN; c += 8) f[c] = __float2bfloat16(0.f);
+        if (tid < MH * 2) S.W4[tid] = P[OFF_W4 + tid];
     }
     __syncthreads();
-    const int m0 = (warp >> 2) * 32, n0 = (warp & 3) * 32;
+    const int m0 = (warp >> 2) * 16, n0 = (warp & 3) * 32;
     const bf16 *WT[3] = {PB + BOFF_W1T, PB + BOFF_W2T, PB + BOFF_W3T};
     const bf16 *Wb[3] = {nullptr, PB + BOFF_W2, PB + BOFF_W3};
     const float *bias[3] = {P + OFF_B1, P + OFF_B2, P + OFF_B3};
     // forward, layers 1-3
+#pragma unroll 1
     for (int L = 0; L < 3; L++) {
-        float acc[2][4][4];
-        zero_acc<32, 32>(acc);
-        if (L == 0) warp_gemm<32, 32, false, true>(S.F, LDF, WT[0], MFIN, MFIN, m0, n0, acc);
-        else warp_gemm<32, 32, false, true>(S.H[L - 1], LDH, WT[L], MH, MH, m0, n0, acc);
-        hidden_epilogue<32, 32>(acc, m0, n0, bias[L], S.Z[L], S.H[L]);
+        float acc[1][4][4];
+        zero_acc<16, 32>(acc);
+        if (L == 0) warp_gemm<16, 32, false, true>(S.F, LDF, WT[0], MFIN, MFIN, m0, n0, acc);
+        else warp_gemm<16, 32, false, true>(S.H[L - 1], LDH, WT[L], MH, MH, m0, n0, acc);
+        hidden_epilogue<16, 32>(acc, m0, n0, bias[L], S.Z[L], S.H[L]);
         __syncthreads();
     }
-    // output layer (fp32), loss, dy
-    if (threadIdx.x < TT * 2) {
-        const int r = threadIdx.x >> 1, c = threadIdx.x & 1;
-        float y = P[OFF_B4 + c];
-        for (int k = 0; k < MH; k++) y += __bfloat162float(S.H[2][r * LDH + k]) * P[OFF_W4 + k * 2 + c];
-        const int i = row0 + r;
-        float dy = 0.f;
+    {  // output layer (fp32), loss, dy: four lanes an output, each every fourth input
+        const int o = tid >> 2, r = o >> 1, c = o & 1, i = row0 + r;
+        float y = 0.f;
+#pragma unroll 8
+        for (int k = tid & 3; k < MH; k += 4) y += __bfloat162float(S.H[2][r * LDH + k]) * S.W4[k * 2 + c];
+        y += __shfl_xor_sync(0xffffffffu, y, 1);
+        y += __shfl_xor_sync(0xffffffffu, y, 2);
+        y += P[OFF_B4 + c];
+        float dy = 0.f, l = 0.f;
         if (i < n) {
             const float2 tg = target[i];
-            const float tv = (c == 0 ? tg.x : tg.y) * inv_scale;
-            const float d = y - tv;
-            atomicAdd(loss, d * d * inv_n);
+            const float d = y - (c == 0 ? tg.x : tg.y) * inv_scale;
+            l = d * d * inv_n;
             dy = 2.f * d * inv_n;
         }
-        S.Y[r * 2 + c] = dy;
+        if ((tid & 3) == 0) S.Y[o] = dy;
+        else l = 0.f;
+        for (int d = 16; d > 0; d >>= 1) l += __shfl_xor_sync(0xffffffffu, l, d);
+        if (lane == 0) S.loss[warp] = l;
     }
     __syncthreads();
-    // dW4, db4
-    if (threadIdx.x < MH * 2) {
-        const int k = threadIdx.x >> 1, c = threadIdx.x & 1;
-        float s = 0.f;
-        for (int r = 0; r < TT; r++) s += __bfloat162float(S.H[2][r * LDH + k]) * S.Y[r * 2 + c];
-        atomicAdd(grad + OFF_W4 + k * 2 + c, s);
+    if (tid == 0) {
+        float l = 0.f;
+        for (int k = 0; k < kTrainThreads / 32; k++) l += S.loss[k];
+        atomicAdd(loss, l);
     }
-    if (threadIdx.x < 2) {
+    {  // dW4, db4: two lanes an output, half the samples each
+        const int o = tid >> 1, k = o >> 1, c = o & 1;
         float s = 0.f;
-        for (int r = 0; r < TT; r++) s += S.Y[r * 2 + threadIdx.x];
-        atomicAdd(grad + OFF_B4 + threadIdx.x, s);
+#pragma unroll 8
+        for (int r = tid & 1; r < TT; r += 2) s += __bfloat162float(S.H[2][r * LDH + k]) * S.Y[r * 2 + c];
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if ((tid & 1) == 0) atomicAdd(grad + OFF_W4 + o, s);
+        if (tid < 2) {
+            float b = 0.f;
+            for (int r = 0; r < TT; r++) b += S.Y[r * 2 + tid];
+            atomicAdd(grad + OFF_B4 + tid, b);
+        }
     }
     __syncthreads();
     // dz3 = (dy W4^T) * silu'(z3): fp32 into Z[2], bf16 into H[2]
-    for (int e = threadIdx.x; e < TT * MH; e += blockDim.x) {
+    for (int e = tid; e < TT * MH; e += kTrainThreads) {
         const int r = e / MH, k = e % MH;
-        const float dh = S.Y[r * 2] * P[OFF_W4 + k * 2] + S.Y[r * 2 + 1] * P[OFF_W4 + k * 2 + 1];
+        const float dh = S.Y[r * 2] * S.W4[k * 2] + S.Y[r * 2 + 1] * S.W4[k * 2 + 1];
         const float dz = dh * dsilu_f(S.Z[2][r * LDZ + k]);
         S.Z[2][r * LDZ + k] = dz;
         S.H[2][r * LDH + k] = __float2bfloat16(dz);
     }
     __syncthreads();
     // layers 3, 2, 1 backward
+#pragma unroll 1
     for (int L = 2; L >= 0; L--) {
-        const bf16 *Hin = L == 0 ? S.F : S.H[L - 1];
-        const int ldin = L == 0 ? LDF : LDH;
-        const int fin = L == 0 ? MFIN : MH;
-        const int woff = L == 0 ? OFF_W1 : (L == 1 ? OFF_W2 : OFF_W3);
-        const int boff = L == 0 ? OFF_B1 : (L == 1 ? OFF_B2 : OFF_B3);
         // dW = Hin^T * dZ  (fin x 128, K = TT)
-        if (fin == MH) {
-            float acc[4][4][4];
-            zero_acc<64, 32>(acc);
-            const int wm0 = (warp >> 2) * 64, wn0 = (warp & 3) * 32;
-            warp_gemm<64, 32, true, false>(Hin, ldin, S.H[L], LDH, TT, wm0, wn0, acc);
-            const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-            for (int mi = 0; mi < 4; mi++)
-#pragma unroll
-                for (int ni = 0; ni < 4; ni++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const int r = wm0 + mi * 16 + g + 8 * (e >> 1);
-                        const int c = wn0 + ni * 8 + 2 * t + (e & 1);
-                        atomicAdd(grad + woff + r * MH + c, acc[mi][ni][e]);
-                    }
+        if (L > 0) {
+            float acc[2][4][4];
+            zero_acc<32, 32>(acc);
+            const int wm0 = (warp >> 2) * 32;
+            warp_gemm<32, 32, true, false>(S.H[L - 1], LDH, S.H[L], LDH, TT, wm0, n0, acc);
+            add_weight_grad<32, 32>(acc, grad + (L == 1 ? OFF_W2 : OFF_W3), wm0, n0, MH);
         } else {
-            float acc[1][4][4];
-            zero_acc<16, 32>(acc);
-            const int wm0 = (warp >> 2) * 16, wn0 = (warp & 3) * 32;
-            warp_gemm<16, 32, true, false>(Hin, ldin, S.H[L], LDH, TT, wm0, wn0, acc);
-            const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-            for (int ni = 0; ni < 4; ni++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int r = wm0 + g + 8 * (e >> 1);
-                    const int c = wn0 + ni * 8 + 2 * t + (e & 1);
-                    if (r < MNFEAT) atomicAdd(grad + woff + r * MH + c, acc[0][ni][e]);
-                }
+            float acc[1][2][4];
+            zero_acc<16, 16>(acc);
+            const int wm0 = (warp >> 3) * 16, wn0 = (warp & 7) * 16;
+            warp_gemm<16, 16, true, false>(S.F, LDF, S.H[0], LDH, TT, wm0, wn0, acc);
+            add_weight_grad<16, 16>(acc, grad + OFF_W1, wm0, wn0, MNFEAT);
         }
-        // db
-        if (threadIdx.x < MH) {
+        {  // db: four lanes a column
+            const int c = tid >> 2;
             float s = 0.f;
-            for (int r = 0; r < TT; r++) s += S.Z[L][r * LDZ + threadIdx.x];
-            atomicAdd(grad + boff + threadIdx.x, s);
+#pragma unroll 8
+            for (int r = tid & 3; r < TT; r += 4) s += S.Z[L][r * LDZ + c];
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if ((tid & 3) == 0) atomicAdd(grad + (L == 0 ? OFF_B1 : (L == 1 ? OFF_B2 : OFF_B3)) + c, s);
         }
         if (L == 0) break;
         // dH_{L-1} = dZ_L * W_L^T, then dZ_{L-1} = dH * silu'(Z_{L-1})
-        float acc[2][4][4];
-        zero_acc<32, 32>(acc);
-        warp_gemm<32, 32, false, true>(S.H[L], LDH, Wb[L], MH, MH, m0, n0, acc);
+        float acc[1][4][4];
+        zero_acc<16, 32>(acc);
+        warp_gemm<16, 32, false, true>(S.H[L], LDH, Wb[L], MH, MH, m0, n0, acc);
         __syncthreads();  // everyone is done reading H[L-1] (dW) and H[L] (this GEMM)
-        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+        const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-        for (int mi = 0; mi < 2; mi++)
+        for (int ni = 0; ni < 4; ni++)
 #pragma unroll
-            for (int ni = 0; ni < 4; ni++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int r = m0 + mi * 16 + g + 8 * h;
-                    const int c = n0 + ni * 8 + 2 * t;
-                    float *z = S.Z[L - 1] + r * LDZ + c;
-                    const float d0 = acc[mi][ni][2 * h] * dsilu_f(z[0]);
-                    const float d1 = acc[mi][ni][2 * h + 1] * dsilu_f(z[1]);
-                    z[0] = d0;
-                    z[1] = d1;
-                    *reinterpret_cast<uint32_t *>(S.H[L - 1] + r * LDH + c) =
-                        pack_bf16(__float2bfloat16(d0), __float2bfloat16(d1));
-                }
+            for (int h = 0; h < 2; h++) {
+                const int r = m0 + g + 8 * h;
+                const int c = n0 + ni * 8 + 2 * t;
+                float2 *z = reinterpret_cast<float2 *>(S.Z[L - 1] + r * LDZ + c);
+                const float d0 = acc[0][ni][2 * h] * dsilu_f(z->x);
+                const float d1 = acc[0][ni][2 * h + 1] * dsilu_f(z->y);
+                *z = make_float2(d0, d1);
+                *reinterpret_cast<uint32_t *>(S.H[L - 1] + r * LDH + c) =
+                    pack_bf16(__float2bfloat16(d0), __float2bfloat16(d1));
+            }
         __syncthreads();
     }
 }
@@ -937,7 +973,7 @@ void launch_mlp_grad(cudaStream_t s, const float *P, const void *PB, const float
 {
     const size_t sm = sizeof(TrainSmem);
     cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    mlp_grad_kernel<<<(n + TT - 1) / TT, 256, sm, s>>>(P, (const bf16 *)PB, in, target, n, ksize, inv_wmax,
+    mlp_grad_kernel<<<(n + TT - 1) / TT, kTrainThreads, sm, s>>>(P, (const bf16 *)PB, in, target, n, ksize, inv_wmax,
                                                        inv_scale, grad, loss);
 }
 
