@@ -58,39 +58,38 @@ int sturm_count(const std::vector<double> &d, const std::vector<double> &e, doub
     return count;
 }
 
-// Solve (T - sigma I) y = b for tridiagonal T, Gaussian elimination with
-// partial pivoting on the dense band (a small system: ~2c + 40 unknowns).
+// Solve (T - sigma I) y = b for tridiagonal T: elimination with partial pivoting,
+// which fills one diagonal above the two.
 void shifted_solve(const std::vector<double> &d, const std::vector<double> &e, double sigma,
                    const std::vector<double> &b, std::vector<double> &y)
 {
     const int n = (int)d.size();
-    std::vector<double> a((size_t)n * n, 0.0), r(b);
+    std::vector<double> p0(n), p1(n, 0.0), p2(n, 0.0), r(b);
     for (int i = 0; i < n; i++) {
-        a[(size_t)i * n + i] = d[i] - sigma;
-        if (i + 1 < n) a[(size_t)i * n + i + 1] = a[(size_t)(i + 1) * n + i] = e[i];
+        p0[i] = d[i] - sigma;
+        if (i + 1 < n) p1[i] = e[i];
     }
-    for (int col = 0; col < n; col++) {
-        int piv = col;
-        for (int i = col + 1; i < n; i++)
-            if (std::fabs(a[(size_t)i * n + col]) > std::fabs(a[(size_t)piv * n + col])) piv = i;
-        if (piv != col) {
-            for (int j = 0; j < n; j++) std::swap(a[(size_t)col * n + j], a[(size_t)piv * n + j]);
-            std::swap(r[col], r[piv]);
+    for (int i = 0; i + 1 < n; i++) {
+        double below = e[i];  // row i + 1: below, p0, p1 at columns i, i + 1, i + 2
+        if (std::fabs(below) > std::fabs(p0[i])) {
+            std::swap(below, p0[i]);
+            std::swap(p0[i + 1], p1[i]);
+            std::swap(p1[i + 1], p2[i]);
+            std::swap(r[i], r[i + 1]);
         }
-        double p = a[(size_t)col * n + col];
-        if (p == 0.0) p = a[(size_t)col * n + col] = 1e-300;  // exactly singular: any scaled eigenvector will do
-        for (int i = col + 1; i < n; i++) {
-            const double f = a[(size_t)i * n + col] / p;
-            if (f == 0.0) continue;
-            for (int j = col; j < n; j++) a[(size_t)i * n + j] -= f * a[(size_t)col * n + j];
-            r[i] -= f * r[col];
-        }
+        if (p0[i] == 0.0) p0[i] = 1e-300;  // exactly singular: any scaled eigenvector will do
+        const double f = below / p0[i];
+        p0[i + 1] -= f * p1[i];
+        p1[i + 1] -= f * p2[i];
+        r[i + 1] -= f * r[i];
     }
+    if (p0[n - 1] == 0.0) p0[n - 1] = 1e-300;
     y.assign(n, 0.0);
     for (int i = n - 1; i >= 0; i--) {
         double s = r[i];
-        for (int j = i + 1; j < n; j++) s -= a[(size_t)i * n + j] * y[j];
-        y[i] = s / a[(size_t)i * n + i];
+        if (i + 1 < n) s -= p1[i] * y[i + 1];
+        if (i + 2 < n) s -= p2[i] * y[i + 2];
+        y[i] = s / p0[i];
     }
 }
 
@@ -107,7 +106,9 @@ std::vector<double> pswf_coefficients(double c)
         lo = std::fmin(lo, d[i] - r);
         hi = std::fmax(hi, d[i] + r);
     }
-    for (int it = 0; it < 200 && hi - lo > 1e-15 * std::fmax(1.0, std::fabs(lo) + std::fabs(hi)); it++) {
+    // to 1e-9 of the interval's scale: the next eigenvalue is about 4c away, so each
+    // inverse iteration gains seven digits or more and six are plenty
+    for (int it = 0; it < 200 && hi - lo > 1e-9 * std::fmax(1.0, std::fabs(lo) + std::fabs(hi)); it++) {
         const double mid = 0.5 * (lo + hi);
         if (sturm_count(d, e, mid) >= 1) hi = mid;
         else lo = mid;
@@ -124,28 +125,29 @@ std::vector<double> pswf_coefficients(double c)
     return x;
 }
 
-// psi_0(c, x) / psi_0(c, 0) from the coefficients, by the Legendre recurrence.
-double pswf_value(const std::vector<double> &coef, double x)
+// psi_0(c, x) / psi_0(c, 0) from the coefficients at n points, by the Legendre
+// recurrence, all points a degree at a time (the divisions go side by side).
+void pswf_values(const std::vector<double> &coef, const double *x, int64_t n, double *out)
 {
-    double p_prev = 1.0, p_cur = x;  // P_0, P_1
-    double out = coef[0] * std::sqrt(0.5), at0 = coef[0] * std::sqrt(0.5);
-    double q_prev = 1.0, q_cur = 0.0;  // the same at x = 0
-    int deg = 1;
-    for (size_t j = 1; j < coef.size(); j++) {
-        const int k = 2 * (int)j;
-        while (deg < k) {
-            const double p_next = ((2 * deg + 1) * x * p_cur - deg * p_prev) / (deg + 1);
-            const double q_next = (-(double)deg * q_prev) / (deg + 1);
-            p_prev = p_cur;
-            p_cur = p_next;
-            q_prev = q_cur;
-            q_cur = q_next;
-            deg++;
+    double at0 = coef[0] * std::sqrt(0.5), q_prev = 1.0, q_cur = 0.0;  // the sum at x = 0; P_0 and P_1 there
+    std::vector<double> p_prev(n, 1.0), p_cur(x, x + n);
+    for (int64_t i = 0; i < n; i++) out[i] = coef[0] * std::sqrt(0.5);
+    for (int deg = 1; deg < 2 * (int)coef.size() - 2; deg++) {
+        for (int64_t i = 0; i < n; i++) {
+            const double p_next = ((2 * deg + 1) * x[i] * p_cur[i] - deg * p_prev[i]) / (deg + 1);
+            p_prev[i] = p_cur[i];
+            p_cur[i] = p_next;
         }
-        out += coef[j] * std::sqrt(k + 0.5) * p_cur;
-        at0 += coef[j] * std::sqrt(k + 0.5) * q_cur;
+        const double q_next = (-(double)deg * q_prev) / (deg + 1);
+        q_prev = q_cur;
+        q_cur = q_next;
+        if (deg % 2) {  // p_cur is the even degree deg + 1
+            const double c = coef[(deg + 1) / 2], norm = std::sqrt(deg + 1 + 0.5);
+            for (int64_t i = 0; i < n; i++) out[i] += c * norm * p_cur[i];
+            at0 += c * norm * q_cur;
+        }
     }
-    return out / at0;
+    for (int64_t i = 0; i < n; i++) out[i] /= at0;
 }
 
 // The sums, folded. The screen is even in l and in m, so with i' = i - M/2 a
@@ -333,10 +335,11 @@ rg_status rg_pswf0(double c, const double *x, int64_t n, double *out)
     if (n < 0 || (n > 0 && (!x || !out))) return fail(RG_ERR_INVALID_ARGUMENT, "x and out must be non-NULL");
     if (!(c > 0.0) || !std::isfinite(c) || c > 1000.0) return fail(RG_ERR_INVALID_ARGUMENT, "c must be in (0, 1000]");
     const std::vector<double> coef = pswf_coefficients(c);
-    for (int64_t k = 0; k < n; k++) {
+    for (int64_t k = 0; k < n; k++)
         if (!(std::fabs(x[k]) <= 1.0)) return fail(RG_ERR_INVALID_ARGUMENT, "x must lie in [-1, 1]");
-        out[k] = pswf_value(coef, x[k]);
-    }
+    std::vector<double> values((size_t)n);  // out may be x
+    pswf_values(coef, x, n, values.data());
+    std::copy(values.begin(), values.end(), out);
     return RG_OK;
 }
 
@@ -358,8 +361,11 @@ rg_status rg_wkern_generate(rg_context *ctx, double theta, const double *w_plane
     RG_CUDA(cudaSetDevice(ctx->device));
     begin_call(ctx);
     const std::vector<double> coef = pswf_coefficients(cc);
-    std::vector<double> taper(M);
-    for (int i = 0; i < M; i++) taper[i] = pswf_value(coef, 2.0 * (double)(i - M / 2) / M);
+    // the taper is even, bit for bit: half of it computed, the rest mirrored
+    std::vector<double> taper(M), half(M / 2 + 1), at(M / 2 + 1);
+    for (int i = 0; i <= M / 2; i++) at[i] = 2.0 * (double)i / M;
+    pswf_values(coef, at.data(), M / 2 + 1, half.data());
+    for (int i = 0; i < M; i++) taper[i] = half[i < M / 2 ? M / 2 - i : i - M / 2];
     const int S = size, ov = oversampling, Q = ov * S;
     const int64_t ntaps = (int64_t)plane_count * Q * Q;
     const int J = M / 2 + 1, K = M / 2 + 2;
