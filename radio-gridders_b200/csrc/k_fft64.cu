@@ -194,38 +194,45 @@ void launch_fft64_2d(cudaStream_t s, double2 *data, int batch, const Fft64Plan &
                              StCols{data, nx, (int64_t)ny * nx});
 }
 
-// Rows of the dirty image: line 2p is grid row p and line 2p + 1 its mirror
-// N - p (pair 0: rows 0 and N/2), so the two rows of a hermitian pair are read
-// at the same time and the second read of each comes from L2. The point read
-// is the hermitian sum of src/reference/grid.c:639-662 (linear index i >= N + 1
-// pairs with N^2 + N - i; row 0 and element (1, 0) are left as they are) at
-// the shifted column (grid.c:665-680); the row goes to its shifted place.
+// Rows of the dirty image: row y of the hermitian sum h (src/reference/grid.c:
+// 639-662: linear index i >= N + 1 pairs with N^2 + N - i; row 0 and element
+// (1, 0) are left as they are) with its columns shifted (grid.c:665-680),
+// f_y[n] = h(y, n + N/2 mod N). Only rows 0..N/2 are transformed: away from column 0,
+// h(N - y, N - x) = conj(h(y, x)), so with d_y = conj(h(N - y, 0)) - h(y, 0), which the
+// thread that reads column 0 leaves in delta,
+//   X_(N-y)[k] = conj(X_y[k] + (-1)^k d_y).
 struct LdImageRow {
     const double2 *g;
+    double2 *delta;
     int N;
-    __device__ int row(int line) const
+    __device__ double2 sum(int64_t i) const
     {
-        const int p = line >> 1;
-        return line & 1 ? (p == 0 ? N / 2 : N - p) : p;
-    }
-    __device__ double2 operator()(int, int line, int n) const
-    {
-        const int y = row(line), x = n < N / 2 ? n + N / 2 : n - N / 2;
-        const int64_t i = (int64_t)y * N + x;
         const double2 a = g[i];
         if (i < N + 1) return a;
         const double2 b = g[(int64_t)N * N + N - i];
         return make_double2(a.x + b.x, a.y - b.y);
     }
-};
-struct StImageRow {
-    double2 *tmp;
-    int N;
-    __device__ void operator()(int, int line, int n, double2 v) const
+    __device__ double2 operator()(int, int y, int n) const
     {
-        const int p = line >> 1;
-        const int y = line & 1 ? (p == 0 ? N / 2 : N - p) : p;
-        tmp[(int64_t)(y < N / 2 ? y + N / 2 : y - N / 2) * N + n] = v;
+        const int x = n < N / 2 ? n + N / 2 : n - N / 2;
+        const double2 h = sum((int64_t)y * N + x);
+        if (x == 0 && y > 0 && y < N / 2) {
+            const double2 m = sum((int64_t)(N - y) * N);
+            delta[y] = make_double2(m.x - h.x, -m.y - h.y);
+        }
+        return h;
+    }
+};
+// Columns of all rows, in shifted order, from the transformed half.
+struct LdImageCol {
+    const double2 *rows, *delta;
+    int N;
+    __device__ double2 operator()(int, int k, int n) const
+    {
+        const int y = n < N / 2 ? n + N / 2 : n - N / 2;
+        if (y <= N / 2) return rows[(int64_t)y * N + k];
+        const double2 v = rows[(int64_t)(N - y) * N + k], d = __ldg(delta + N - y);
+        return k & 1 ? make_double2(v.x - d.x, d.y - v.y) : make_double2(v.x + d.x, -v.y - d.y);
     }
 };
 // Columns: the transformed grid and the image at their shifted places.
@@ -247,8 +254,9 @@ void launch_image_from_grid(cudaStream_t s, double2 *grid, double2 *tmp, double 
                             const Fft64Plan &p)
 {
     const int N = p.n;
-    launch_fft64_lines<false>(s, p, 1, N, -1, LdImageRow{grid, N}, StImageRow{tmp, N});
-    launch_fft64_lines<true>(s, p, 1, N, -1, LdCols{tmp, N, 0}, StImageCol{grid, image, taper, N});
+    double2 *delta = tmp + (int64_t)(N / 2 + 1) * N;
+    launch_fft64_lines<false>(s, p, 1, N / 2 + 1, -1, LdImageRow{grid, delta, N}, StRows{tmp, N});
+    launch_fft64_lines<true>(s, p, 1, N, -1, LdImageCol{tmp, delta, N}, StImageCol{grid, image, taper, N});
 }
 
 }  // namespace rg

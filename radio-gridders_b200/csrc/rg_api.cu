@@ -1309,7 +1309,7 @@ rg_status rg_image_from_grid(rg_context *ctx, double *uvgrid, int grid_size, dou
     OutView g;
     RG_CHECK(out_view(ctx, uvgrid, sizeof(double2) * (size_t)cells, "img_grid", true, &g));
     void *tmp;
-    RG_CHECK(scratch(ctx, "img_tmp", sizeof(double2) * (size_t)cells, &tmp));
+    RG_CHECK(scratch(ctx, "img_tmp", sizeof(double2) * (size_t)(N / 2 + 1) * (N + 1), &tmp));
     const void *taper = nullptr;
     if (taper_1d) RG_CHECK(stage_in(ctx, taper_1d, sizeof(double) * N, "img_taper", &taper));
     OutView img;

@@ -240,7 +240,7 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out);
 void launch_fft64_2d(cudaStream_t s, double2 *data, int batch, const Fft64Plan &py, const Fft64Plan &px, int sign);
 // The dirty image of an n x n grid (n even): hermitian sum, shift, transform
 // (sign -1), shift; the result goes to grid and its real part, over
-// taper[y] taper[x] if given, to image. tmp: n x n.
+// taper[y] taper[x] if given, to image. tmp: (n/2 + 1) (n + 1) elements.
 void launch_image_from_grid(cudaStream_t s, double2 *grid, double2 *tmp, double *image, const double *taper,
                             const Fft64Plan &p);
 
