@@ -53,8 +53,10 @@ __device__ __forceinline__ int div_nonneg(int a, int d, float inv)
 // capacity) nothing is written, so the caller can rerun on the same grid.  In
 // a batch (poison != nullptr) an overflow also stops the later passes' writes
 // until the batch reruns them.
-constexpr int kAddBackRows = 4;
-
+// ROWS rows a thread: four, so a column's tower range is found once for them
+// (2048 x 2048: 32 against 37 us), but one on grids up to 1024, whose CTAs would
+// not fill the device (512 x 512: 11.6 -> 6.6 us).
+template <int ROWS>
 __global__ void add_back_kernel(const float2 *__restrict__ subimg, const int *__restrict__ tower_count,
                                 double2 *__restrict__ master, int N, int S, int M, int chunk,
                                 int nchunk, int overwrite, const int *__restrict__ range,
@@ -75,11 +77,10 @@ __global__ void add_back_kernel(const float2 *__restrict__ subimg, const int *__
     // S is a power of two, so 1 / S^2 is exact and multiplying by it gives
     // the quotient the division would, bit for bit
     const double inv_norm = 1.0 / (double)(S * S);
-    // kAddBackRows rows per thread, blockDim.y apart (the column's tower range
-    // is found once)
-    const int gy_end = min(N, (int)(blockIdx.y + 1) * (int)blockDim.y * kAddBackRows);
+    // the rows are blockDim.y apart
+    const int gy_end = min(N, (int)(blockIdx.y + 1) * (int)blockDim.y * ROWS);
 #pragma unroll 1
-    for (int gy = blockIdx.y * blockDim.y * kAddBackRows + threadIdx.y; gy < gy_end; gy += blockDim.y) {
+    for (int gy = blockIdx.y * blockDim.y * ROWS + threadIdx.y; gy < gy_end; gy += blockDim.y) {
         const int ay = gy + M / 2;
         int cy_hi = div_nonneg(ay, chunk, inv);
         const int cy_lo = (ay - S) >= 0 ? div_nonneg(ay - S, chunk, inv) + 1 : 0;
@@ -108,9 +109,13 @@ void launch_add_back(cudaStream_t s, const float2 *subimg, const int *tower_coun
                      const int *range, const int *counts, int slot_cap, int group_cap, int *poison)
 {
     dim3 blk(32, 8);
-    dim3 grd((grid_size + 31) / 32, (grid_size + 8 * kAddBackRows - 1) / (8 * kAddBackRows));
-    add_back_kernel<<<grd, blk, 0, s>>>(subimg, tower_count, master, grid_size, subgrid, margin,
-                                        chunk, nchunk, overwrite, range, counts, slot_cap, group_cap, poison);
+    auto go = [&](auto kernel, int rows) {
+        dim3 grd((grid_size + 31) / 32, (grid_size + 8 * rows - 1) / (8 * rows));
+        kernel<<<grd, blk, 0, s>>>(subimg, tower_count, master, grid_size, subgrid, margin, chunk, nchunk, overwrite,
+                                   range, counts, slot_cap, group_cap, poison);
+    };
+    if (grid_size > 1024) go(add_back_kernel<4>, 4);
+    else go(add_back_kernel<1>, 1);
 }
 
 }  // namespace rg
