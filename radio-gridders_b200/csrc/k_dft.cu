@@ -233,7 +233,7 @@ __device__ __forceinline__ double turns(double a, double b, double c)
 // MIN..MAX moments only. part: [share][row][column].
 // Bound by the FP64 pipe: 2 J + about 2 multiply-adds a pixel and visibility,
 // where reduction and sincospi took about 59. 500 x 500 pixels, 20,000
-// visibilities: 15.9 -> 3.6 ms.
+// visibilities: 15.9 -> 3.5 ms.
 constexpr int kDftVis = 32, kDftStrideB = TILE + 4;  // 4 mod 16: a fragment's 4 k x 8 rows on distinct banks
 
 template <int MIN, int MAX>
@@ -356,13 +356,14 @@ __global__ void dft_shares_kernel(const double *part, int shares, double *image,
     }
 }
 
-// Shares the visibilities are split into: about six resident rounds of CTAs over
-// the whole image's tiles, at least 512 visibilities each. The whole image's, so
+// Shares the visibilities are split into: six rounds of four resident CTAs an SM
+// over the whole image's tiles, for a short tail (three rounds: 3.64 against 3.48
+// ms at 500 x 500), at least 512 visibilities each. The whole image's, so
 // a band of rows is summed as the image's rows are.
 int dft64_shares(int grid_size, int64_t n, int sm_count)
 {
     const int64_t tiles = (int64_t)((grid_size + TILE - 1) / TILE) * ((grid_size + TILE - 1) / TILE);
-    int64_t s = ((int64_t)sm_count * 12 + tiles - 1) / tiles;
+    int64_t s = ((int64_t)sm_count * 24 + tiles - 1) / tiles;
     if (s > n / 512) s = n / 512;
     return s < 1 ? 1 : (int)(s > 64 ? 64 : s);
 }
