@@ -128,7 +128,15 @@ rg_status roots64(rg_context *ctx, int n, const double2 **out)
     const bool fresh = known == ctx->scratch.end() || !known->second.ptr;
     void *mem;
     RG_CHECK(scratch(ctx, name.c_str(), sizeof(double2) * (size_t)n, &mem));
-    if (fresh) fft64_twiddle_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>((double2 *)mem, n);
+    if (fresh) {
+        fft64_twiddle_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>((double2 *)mem, n);
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);  // a later call may be on another stream
+        if (e != cudaSuccess) {
+            cudaFree(mem);
+            ctx->scratch.erase(name);
+            return cuda_fail(e, "table of roots");
+        }
+    }
     *out = (const double2 *)mem;
     return RG_OK;
 }
@@ -181,6 +189,7 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
         p.chirp = chirp;
     }
     RG_CUDA(cudaGetLastError());
+    RG_CUDA(cudaStreamSynchronize(ctx->stream));  // a later call may be on another stream
     ctx->fft64_plans[n] = p;
     *out = p;
     return RG_OK;
