@@ -162,33 +162,46 @@ void pswf_values(const std::vector<double> &coef, const double *x, int64_t n, do
 // The products run on the FP64 tensor pipe (mma m8n8k4, 37 TFLOP/s measured, the
 // rate of the FP64 multiply-add pipe, with an eighth of its instructions and
 // operand reads): 64 x 64 tiles, K in shared memory 68 deep (all of the default
-// screen's 66), one 32 x 32 block a warp. Bound by that pipe: 2.6 GFLOP for
-// 401 planes of 16 x 16 taps, 8 x oversampled. The call: 4831 -> 374 us
-// (the sums as plain loops took 3387 and 1152 us).
+// screen's 66), one 32 x 32 block a warp. 401 planes of 16 x 16 taps, 8 x
+// oversampled (2.6 GFLOP): 38 + 80 us, two thirds of that pipe's rate; copies and
+// stores by running pointers and offsets in place of an index for each element
+// took them there from 41 + 93 us, at half the instructions. Persistent CTAs
+// with the factors resident and the other operand double-buffered (two CTAs an
+// SM) take 43 + 84, four or five CTAs an SM with shallower tiles 37..38 +
+// 78..85. The call: 4831 -> 180 us (the sums as plain loops took 3387 and 1152).
 
 // a[k][row], row = (plane K + j') 2 + part: the screen's rows as the left
 // factor. k < M/2: s(i' = k); k = M/2, M/2 + 1: the edge i' = -M/2 times the
 // edge factors' real and imaginary parts. The rows j' run the same way, the
 // edge row twice, so the second product takes them as they come.
+// A thread takes one pixel of 8 planes, whose root and taper they share: 13 us
+// for 401 planes of 65 x 65 pixels, 20..24 us with an element a thread (bound by
+// instructions issued, 346 -> 135 an element).
+constexpr int kScreenPlanes = 8;
+
 __global__ void wscreen_kernel(const double *__restrict__ w_planes, int planes, const double *__restrict__ taper,
                                int M, double theta, double2 *__restrict__ a)
 {
-    const int h = M / 2, J = h + 1;
-    const int64_t pairs = (int64_t)planes * (h + 2), total = (int64_t)planes * J * J;
-    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < total; n += (int64_t)gridDim.x * blockDim.x) {
-        const int j = (int)(n % J), p = (int)((n / J) % planes), k = (int)(n / ((int64_t)J * planes));
+    const int h = M / 2, J = h + 1, k = blockIdx.y;
+    const int64_t pairs = (int64_t)planes * (h + 2);
+    const unsigned groups = (planes + kScreenPlanes - 1) / kScreenPlanes, total = groups * J;  // below 2^25
+    for (unsigned n = blockIdx.x * blockDim.x + threadIdx.x; n < total; n += gridDim.x * blockDim.x) {
+        const int j = n % J;
         const int ic = k < h ? k : -h, jc = j < h ? j : -h;
         const double l = theta * (double)ic / M, m = theta * (double)jc / M;
         const double one_minus_n = 1.0 - sqrt(1.0 - (l * l + m * m));
-        double sn, cs;
-        sincospi(2.0 * w_planes[p] * one_minus_n, &sn, &cs);
-        const double t = taper[ic + h] * taper[jc + h], re = t * cs, im = t * sn;
-        double2 *at = a + (int64_t)k * pairs + (int64_t)p * (h + 2) + j;
-        at[0] = make_double2(re, im);
-        if (k == h) at[pairs] = make_double2(-im, re);
-        if (j == h) {
-            at[1] = make_double2(-im, re);
-            if (k == h) at[pairs + 1] = make_double2(-re, -im);
+        const double t = taper[ic + h] * taper[jc + h];
+        for (int p = n / J; p < planes; p += groups) {
+            double sn, cs;
+            sincospi(2.0 * w_planes[p] * one_minus_n, &sn, &cs);
+            const double re = t * cs, im = t * sn;
+            double2 *at = a + (int64_t)k * pairs + (int64_t)p * (h + 2) + j;
+            at[0] = make_double2(re, im);
+            if (k == h) at[pairs] = make_double2(-im, re);
+            if (j == h) {
+                at[1] = make_double2(-im, re);
+                if (k == h) at[pairs + 1] = make_double2(-re, -im);
+            }
         }
     }
 }
@@ -214,30 +227,52 @@ __device__ __forceinline__ void mma_f64(double2 &c, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// 16 bytes to shared memory, or zeros where !on
-__device__ __forceinline__ void cp_async16_if(void *smem, const void *gmem, bool on)
+// 16 bytes to shared memory, or zeros where bytes is 0
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int bytes)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
-                 "l"(gmem), "r"(on ? 16 : 0)
+                 "l"(gmem), "r"(bytes)
                  : "memory");
 }
 
+// A lane's two neighbouring columns of an operand: element of depth k at
+// p[k * stride], and nothing where the columns lie past the edge (p then
+// points at the operand's first columns and is not read).
+struct Operand {
+    const double *p;
+    int64_t stride;
+    int bytes;
+    __device__ Operand(const double *base, int64_t off, int64_t stride_, bool on)
+        : p(base + (on ? off : 0)), stride(stride_), bytes(on ? 16 : 0)
+    {
+    }
+};
+
 // One warp's 32 x 32 block of a 64 x 64 tile: rows row0 + 8 i, columns col(j) +
-// 0..7; c[i][j] holds row lane / 4, columns 2 (lane % 4) and the next. a and b
-// give a lane's two neighbouring elements of depth k (a warp copies one depth
-// of both), or nullptr past the edge.
-template <class A, class B, class Col>
-__device__ __forceinline__ void gemm_tile(double2 (&c)[4][4], double *sa, double *sb, int K, A a, B b, int row0, Col col)
+// 0..7; c[i][j] holds row lane / 4, columns 2 (lane % 4) and the next. A warp
+// copies one depth of both operands at a time.
+template <class Col>
+__device__ __forceinline__ void gemm_tile(double2 (&c)[4][4], double *sa, double *sb, int K, Operand a, Operand b,
+                                          int row0, Col col)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int W = kGemmThreads / 32;
+    a.p += warp * a.stride, b.p += warp * b.stride;
     for (int k0 = 0; k0 < K; k0 += kGemmDepth) {
-        const int depth = min(kGemmDepth, (K - k0 + 3) & ~3);
+        const int live = min(kGemmDepth, K - k0), depth = (live + 3) & ~3;
         __syncthreads();
-        for (int k = warp; k < depth; k += kGemmThreads / 32) {
-            const bool live = k0 + k < K;
-            const double *ga = live ? a(k0 + k, 2 * lane) : nullptr, *gb = live ? b(k0 + k, 2 * lane) : nullptr;
-            cp_async16_if(sa + k * kGemmStride + 2 * lane, ga, ga != nullptr);
-            cp_async16_if(sb + k * kGemmStride + 2 * lane, gb, gb != nullptr);
+        double *da = sa + warp * kGemmStride + 2 * lane, *db = sb + warp * kGemmStride + 2 * lane;
+        int k = warp;
+#pragma unroll 4
+        for (; k < live; k += W) {
+            cp_async16(da, a.p, a.bytes);
+            cp_async16(db, b.p, b.bytes);
+            a.p += W * a.stride, b.p += W * b.stride;
+            da += W * kGemmStride, db += W * kGemmStride;
+        }
+        if (k < depth) {  // less than W depths of zeros
+            *(double2 *)da = make_double2(0.0, 0.0);
+            *(double2 *)db = make_double2(0.0, 0.0);
         }
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
         __syncthreads();
@@ -271,8 +306,7 @@ __global__ void __launch_bounds__(kGemmThreads) wkgen_rows_kernel(const double *
     double2 c[4][4] = {};
     gemm_tile(
         c, gemm_sm, gemm_sm + kGemmDepth * kGemmStride, K,
-        [&](int k, int x) { return r0 + x < rows ? a + k * rows + r0 + x : nullptr; },
-        [&](int k, int x) { return q0 + x < Q ? cq + (int64_t)k * Q + q0 + x : nullptr; }, row0,
+        Operand(a, r0 + 2 * lane, rows, r0 + 2 * lane < rows), Operand(cq, q0 + 2 * lane, Q, q0 + 2 * lane < Q), row0,
         [&](int j) { return col0 + 8 * j; });
 #pragma unroll
     for (int i = 0; i < 4; i++)
@@ -300,27 +334,30 @@ __global__ void __launch_bounds__(kGemmThreads) wkgen_cols_kernel(const double *
     const int row0 = (warp >> 1) * 32, col0 = (warp & 1) * 16;
     const double *Tp = T + (int64_t)p * (h + 2) * 2 * Q;
     double2 c[4][4] = {};
+    const int bx = x0 + (2 * lane & 31);
     gemm_tile(
         c, gemm_sm, gemm_sm + kGemmDepth * kGemmStride, h + 2,
-        [&](int k, int x) { return y0 + x < Q ? cq + (int64_t)k * Q + y0 + x : nullptr; },
-        [&](int k, int x) {
-            const int part = x >> 5, q = x0 + (x & 31);
-            return q < Q ? Tp + ((int64_t)k * 2 + part) * Q + q : nullptr;
-        },
-        row0, [&](int j) { return col0 + 8 * (j & 1) + 32 * (j >> 1); });
+        Operand(cq, y0 + 2 * lane, Q, y0 + 2 * lane < Q), Operand(Tp, (lane >> 4) * Q + bx, 2 * Q, bx < Q), row0,
+        [&](int j) { return col0 + 8 * (j & 1) + 32 * (j >> 1); });
     const double inv = 1.0 / ((double)M * M);
+    double2 *o = out + (int64_t)p * Q * Q;
+    int ox[2];  // S is even: a lane's two taps are neighbours
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int j = 0; j < 2; j++) {
+        const int qx = x0 + col0 + 8 * j + 2 * (lane & 3), xf = qx / S;
+        ox[j] = qx < Q ? xf * S * S + qx - xf * S : -1;
+    }
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int qy = y0 + row0 + 8 * i + (lane >> 2), qx = x0 + col0 + 8 * j + 2 * (lane & 3);
-            if (qy < Q && qx < Q) {
-                const int yf = qy / S, ty = qy - yf * S, xf = qx / S, tx = qx - xf * S;  // S is even
-                double2 *o = out + ((((int64_t)p * ov + yf) * ov + xf) * S + ty) * S + tx;
-                o[0] = make_double2(c[i][j].x * inv, c[i][j + 2].x * inv);
-                o[1] = make_double2(c[i][j].y * inv, c[i][j + 2].y * inv);
+    for (int i = 0; i < 4; i++) {
+        const int qy = y0 + row0 + 8 * i + (lane >> 2), yf = qy / S;
+        const int64_t oy = (int64_t)yf * Q * S + (qy - yf * S) * S;
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            if (qy < Q && ox[j] >= 0) {
+                o[oy + ox[j]] = make_double2(c[i][j].x * inv, c[i][j + 2].x * inv);
+                o[oy + ox[j] + 1] = make_double2(c[i][j].y * inv, c[i][j + 2].y * inv);
             }
-        }
+    }
 }
 
 }  // namespace
@@ -381,7 +418,8 @@ rg_status rg_wkern_generate(rg_context *ctx, double theta, const double *w_plane
     RG_CUDA(cudaMemcpyAsync(d_w, w_planes, sizeof(double) * plane_count, cudaMemcpyHostToDevice, ctx->stream));
     RG_CUDA(cudaMemcpyAsync(d_taper, taper.data(), sizeof(double) * M, cudaMemcpyHostToDevice, ctx->stream));
     auto blocks = [](int64_t n) { return (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 32); };
-    wscreen_kernel<<<blocks((int64_t)plane_count * J * J), 256, 0, ctx->stream>>>(
+    const int groups = (plane_count + kScreenPlanes - 1) / kScreenPlanes;
+    wscreen_kernel<<<dim3(blocks((int64_t)groups * J), J), 256, 0, ctx->stream>>>(
         (const double *)d_w, plane_count, (const double *)d_taper, M, theta, (double2 *)d_s);
     wkgen_factors_kernel<<<blocks((int64_t)Q * K), 256, 0, ctx->stream>>>(S, ov, M, (double *)d_cq);
     const int smem = 2 * kGemmDepth * kGemmStride * (int)sizeof(double);
