@@ -4,11 +4,11 @@
 // Both passes are bound by memory and by the latency of one CTA's
 // load - transform - store sequence, with the FP64 pipe behind them
 // (5 n^2 log2 n^2 operations: 0.7 GFLOP at n = 2500). One image of a 2500 x 2500
-// grid, with the caller's copy of the grid: 333 us, against 4522 us as
+// grid, with the caller's copy of the grid: 300 us, against 4522 us as
 // hermitian, shift, radix-2 Bluestein rows, transpose, rows, transpose, shift
-// and real part, each a pass of its own. The rows take 114 us and the columns
-// 157 (193 and 227 with 16 points a thread and 11 warps an SM, strided
-// twiddles and addresses formed point by point).
+// and real part, each a pass of its own. The rows take 77 us (114 with all of
+// them transformed, 193 with 16 points a thread and 11 warps an SM, strided
+// twiddles and addresses formed point by point) and the columns 159 (227).
 #include <algorithm>
 #include <string>
 
