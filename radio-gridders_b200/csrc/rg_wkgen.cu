@@ -126,28 +126,42 @@ std::vector<double> pswf_coefficients(double c)
 }
 
 // psi_0(c, x) / psi_0(c, 0) from the coefficients at n points, by the Legendre
-// recurrence, all points a degree at a time (the divisions go side by side).
+// recurrence, a block of points a degree at a time (the divisions go side by
+// side). Nothing is allocated by n, and out may be x.
 void pswf_values(const std::vector<double> &coef, const double *x, int64_t n, double *out)
 {
-    double at0 = coef[0] * std::sqrt(0.5), q_prev = 1.0, q_cur = 0.0;  // the sum at x = 0; P_0 and P_1 there
-    std::vector<double> p_prev(n, 1.0), p_cur(x, x + n);
-    for (int64_t i = 0; i < n; i++) out[i] = coef[0] * std::sqrt(0.5);
-    for (int deg = 1; deg < 2 * (int)coef.size() - 2; deg++) {
-        for (int64_t i = 0; i < n; i++) {
-            const double p_next = ((2 * deg + 1) * x[i] * p_cur[i] - deg * p_prev[i]) / (deg + 1);
-            p_prev[i] = p_cur[i];
-            p_cur[i] = p_next;
-        }
+    constexpr int B = 512;  // four arrays of 4 KB
+    const int degrees = 2 * (int)coef.size() - 2;
+    std::vector<double> scaled(coef.size());
+    for (size_t j = 0; j < coef.size(); j++) scaled[j] = coef[j] * std::sqrt(2.0 * (double)j + 0.5);
+    double at0 = scaled[0], q_prev = 1.0, q_cur = 0.0;  // the sum at x = 0; P_0 and P_1 there
+    for (int deg = 1; deg < degrees; deg++) {
         const double q_next = (-(double)deg * q_prev) / (deg + 1);
         q_prev = q_cur;
         q_cur = q_next;
-        if (deg % 2) {  // p_cur is the even degree deg + 1
-            const double c = coef[(deg + 1) / 2], norm = std::sqrt(deg + 1 + 0.5);
-            for (int64_t i = 0; i < n; i++) out[i] += c * norm * p_cur[i];
-            at0 += c * norm * q_cur;
-        }
+        if (deg % 2) at0 += scaled[(deg + 1) / 2] * q_cur;
     }
-    for (int64_t i = 0; i < n; i++) out[i] /= at0;
+    double xb[B], p_prev[B], p_cur[B], sum[B];
+    for (int64_t b = 0; b < n; b += B) {
+        const int cnt = (int)std::min<int64_t>(B, n - b);
+        for (int i = 0; i < cnt; i++) {
+            xb[i] = p_cur[i] = x[b + i];
+            p_prev[i] = 1.0;
+            sum[i] = scaled[0];
+        }
+        for (int deg = 1; deg < degrees; deg++) {
+            for (int i = 0; i < cnt; i++) {
+                const double p_next = ((2 * deg + 1) * xb[i] * p_cur[i] - deg * p_prev[i]) / (deg + 1);
+                p_prev[i] = p_cur[i];
+                p_cur[i] = p_next;
+            }
+            if (deg % 2) {  // p_cur is the even degree deg + 1
+                const double c = scaled[(deg + 1) / 2];
+                for (int i = 0; i < cnt; i++) sum[i] += c * p_cur[i];
+            }
+        }
+        for (int i = 0; i < cnt; i++) out[b + i] = sum[i] / at0;
+    }
 }
 
 // The sums, folded. The screen is even in l and in m, so with i' = i - M/2 a
@@ -374,9 +388,7 @@ rg_status rg_pswf0(double c, const double *x, int64_t n, double *out)
     const std::vector<double> coef = pswf_coefficients(c);
     for (int64_t k = 0; k < n; k++)
         if (!(std::fabs(x[k]) <= 1.0)) return fail(RG_ERR_INVALID_ARGUMENT, "x must lie in [-1, 1]");
-    std::vector<double> values((size_t)n);  // out may be x
-    pswf_values(coef, x, n, values.data());
-    std::copy(values.begin(), values.end(), out);
+    pswf_values(coef, x, n, out);
     return RG_OK;
 }
 

@@ -1,5 +1,8 @@
 """The project's synthetic-data and w-kernel generator (CPU)."""
 import importlib
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -64,3 +67,27 @@ def test_library_pswf_matches_generator(c):
     assert np.abs(rg.pswf0(c, x) - sim.pswf0(c, x)).max() < 1e-13
     with pytest.raises(rg.RGError):
         rg.pswf0(c, np.array([1.5]))
+
+
+_PSWF_LOW_MEMORY = """
+import importlib, resource, sys
+import numpy as np
+rg = importlib.import_module("radio-gridders_b200")
+n = 1 << 22
+x = np.linspace(-1.0, 1.0, n)
+out = np.empty(n)
+out[:] = 0.0
+part = rg.pswf0(7.0, x[::4096])
+used = int(next(l for l in open("/proc/self/status") if l.startswith("VmSize")).split()[1]) << 10
+resource.setrlimit(resource.RLIMIT_AS, (used + (16 << 20),) * 2)
+status = rg.lib().rg_pswf0(7.0, x.ctypes.data, n, out.ctypes.data)
+sys.exit(0 if status == 0 and np.array_equal(out[::4096], part) else 1)
+"""
+
+
+def test_native_pswf_needs_no_memory_by_its_points():
+    """Four million points with 16 MB of address space left (their 32 MB are the
+    caller's): an allocation by the number of points would end the process
+    inside the C call. Every point's value is the one it has in a short call."""
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    assert subprocess.run([sys.executable, "-c", _PSWF_LOW_MEMORY], cwd=repo).returncode == 0
