@@ -130,7 +130,9 @@ rg_status roots64(rg_context *ctx, int n, const double2 **out)
     RG_CHECK(scratch(ctx, name.c_str(), sizeof(double2) * (size_t)n, &mem));
     if (fresh) {
         fft64_twiddle_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>((double2 *)mem, n);
-        const cudaError_t e = cudaStreamSynchronize(ctx->stream);  // a later call may be on another stream
+        // a launch that failed shows here alone: the stream has nothing to report
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // a later call may be on another stream
         if (e != cudaSuccess) {
             cudaFree(mem);
             ctx->scratch.erase(name);
