@@ -200,9 +200,16 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
 void launch_fft64_2d(cudaStream_t s, double2 *data, int batch, const Fft64Plan &py, const Fft64Plan &px, int sign)
 {
     const int ny = py.n, nx = px.n;
-    launch_fft64_lines<false>(s, px, 1, batch * ny, sign, LdRows{data, nx}, StRows{data, nx});
-    launch_fft64_lines<true>(s, py, batch, nx, sign, LdCols{data, nx, (int64_t)ny * nx},
-                             StCols{data, nx, (int64_t)ny * nx});
+    const int64_t array = (int64_t)ny * nx;
+    // a launch counts its lines and CTAs in 32 bits: at most 2^30 lines each
+    // (2^31 rows of 2 points are 69 GB, which fits the device)
+    const int step = (1 << 30) / std::max(ny, nx);
+    for (int64_t at = 0; at < batch; at += step) {
+        const int cnt = (int)std::min<int64_t>(step, batch - at);
+        double2 *d = data + at * array;
+        launch_fft64_lines<false>(s, px, 1, cnt * ny, sign, LdRows{d, nx}, StRows{d, nx});
+        launch_fft64_lines<true>(s, py, cnt, nx, sign, LdCols{d, nx, array}, StCols{d, nx, array});
+    }
 }
 
 // Rows of the dirty image: row y of the hermitian sum h (src/reference/grid.c:
