@@ -234,13 +234,14 @@ __global__ void __launch_bounds__(kDirectThreads) wstack_direct_kernel(
     int p0[V];
     double2 acc[V];
     const int64_t first = (int64_t)blockIdx.x * (kDirectThreads * V) + threadIdx.x;
-    unsigned bad = 0;
+    unsigned bad = 0, refused = 0;  // refused: the visibilities with no taps in the stack
     for (int q = 0; q < V; q++) {
         const int64_t i = first + q * kDirectThreads;
         DegridCell c;
         const unsigned e = i < nvis ? degrid_cell(g, u[i], v[i], w[i], c) : DERR_GRID_RANGE;
         const bool ok = e == 0;
         if (i < nvis) bad |= e;
+        if (!ok) refused |= 1u << q;
 #pragma unroll
         for (int t = 0; t < SU; t++) {
             gu[q][t] = ok && t < g.suv ? c.gu[t] : 0.0;
@@ -300,7 +301,8 @@ __global__ void __launch_bounds__(kDirectThreads) wstack_direct_kernel(
     }
     for (int q = 0; q < V; q++) {
         const int64_t i = first + q * kDirectThreads;
-        if (i < nvis) out[i] = acc[q];
+        // zero also where a source's value is infinite and the sum is not a number
+        if (i < nvis) out[i] = refused >> q & 1 ? make_double2(0.0, 0.0) : acc[q];
     }
 }
 

@@ -61,3 +61,21 @@ def test_predict_device_buffers_and_errors(rg, ctx, sim):
     bad["points"] = np.array([[0.9 * c["theta"], 0.0]])  # outside the image
     with pytest.raises(rg.RGError):
         _run(ctx, bad)
+
+
+# a few sources go directly, 3000 through the stack
+@pytest.mark.parametrize("nv,npts", [(200, 3), (30, 3000)])
+def test_refused_visibility_is_zero_beside_an_infinite_source(rg, ctx, sim, nv, npts):
+    """A grid correction of zero makes every source infinite; the visibilities
+    whose taps leave the stack, and those that are not finite, come back as zero
+    with the error all the same, and only those."""
+    c = case(sim, seed=3, lam=1280.0, nv=nv, npts=npts)
+    c["corr_n"] = np.zeros_like(c["corr_n"])
+    c["u"][nv // 2] *= 1e6
+    c["w"][nv - 1] = np.nan
+    out = np.full(nv, 7.0 + 7.0j)
+    with pytest.raises(rg.RGError):
+        _run(ctx, c, out=out)
+    zero = np.zeros(nv, bool)
+    zero[[nv // 2, nv - 1]] = True
+    assert np.all(out[zero] == 0) and not np.isfinite(out[~zero]).any()
