@@ -54,8 +54,10 @@ __device__ __forceinline__ int div_nonneg(int a, int d, float inv)
 // a batch (poison != nullptr) an overflow also stops the later passes' writes
 // until the batch reruns them.
 // ROWS rows a thread: four, so a column's tower range is found once for them
-// (2048 x 2048: 32 against 37 us), but one on grids up to 1024, whose CTAs would
-// not fill the device (512 x 512: 11.6 -> 6.6 us).
+// (2048 x 2048: 32 against 37 us), but one on grids up to 896, whose CTAs would
+// not fill the device. The stage with one and with four, S = 128: 512 x 512 10.6
+// and 14.1 us, 768 12.6 and 14.7, 896 14.7 and 15.0, 1000 16.7 both; S = 512,
+// 1024 x 1024: 16.2 and 15.0.
 template <int ROWS>
 __global__ void add_back_kernel(const float2 *__restrict__ subimg, const int *__restrict__ tower_count,
                                 double2 *__restrict__ master, int N, int S, int M, int chunk,
@@ -114,7 +116,7 @@ void launch_add_back(cudaStream_t s, const float2 *subimg, const int *tower_coun
         kernel<<<grd, blk, 0, s>>>(subimg, tower_count, master, grid_size, subgrid, margin, chunk, nchunk, overwrite,
                                    range, counts, slot_cap, group_cap, poison);
     };
-    if (grid_size > 1024) go(add_back_kernel<4>, 4);
+    if (grid_size > 896) go(add_back_kernel<4>, 4);
     else go(add_back_kernel<1>, 1);
 }
 
