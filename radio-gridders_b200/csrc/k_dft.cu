@@ -89,8 +89,17 @@ __global__ void __launch_bounds__(256) dft_kernel(const double *__restrict__ u,
                                                   double factor, int row0, int nrows,
                                                   const double *__restrict__ wmax)
 {
-    // FP64: only the tiles that the moments do not cover
-    if (MODE == RG_DFT_FP64 && dft_moments(blockIdx.x * TILE, row0 + blockIdx.y * TILE, N, theta, *wmax) > 0) return;
+    // FP64: the tiles that the moments do not cover (wmax nullptr: all), one share
+    // of the visibilities a CTA as the moments have, so a few such tiles do not
+    // leave the device idle
+    int64_t k0 = 0, k1 = nvis;
+    if (MODE == RG_DFT_FP64) {
+        if (wmax && dft_moments(blockIdx.x * TILE, row0 + blockIdx.y * TILE, N, theta, *wmax) > 0) return;
+        const int64_t share = (nvis + gridDim.z - 1) / gridDim.z;
+        k0 = blockIdx.z * share;
+        k1 = min(nvis, k0 + share);
+        image += (int64_t)blockIdx.z * nrows * N;
+    }
     // FP32 modes: (u, v, w, Re V) as one 16-byte entry and Im V beside it, so a
     // visibility is two shared-memory loads in the inner loop
     __shared__ float4 s4[DFT_BATCH];
@@ -120,8 +129,8 @@ __global__ void __launch_bounds__(256) dft_kernel(const double *__restrict__ u,
     }
     double acc[PIX] = {0.0, 0.0, 0.0, 0.0};
 
-    for (int64_t b0 = 0; b0 < nvis; b0 += DFT_BATCH) {
-        const int cnt = (int)(nvis - b0 < DFT_BATCH ? nvis - b0 : DFT_BATCH);
+    for (int64_t b0 = k0; b0 < k1; b0 += DFT_BATCH) {
+        const int cnt = (int)(k1 - b0 < DFT_BATCH ? k1 - b0 : DFT_BATCH);
         __syncthreads();
         if ((int)threadIdx.x < cnt) {
             const int64_t k = b0 + threadIdx.x;
@@ -230,7 +239,7 @@ __device__ __forceinline__ double turns(double a, double b, double c)
 // m8n8k4: the depth is two visibilities' real and imaginary parts). 32
 // visibilities at a time: phasors of both sides into shared memory, then the
 // products; the weights w^j are put on the left fragment in registers. Tiles of
-// MIN..MAX moments only. part: [share][row][column].
+// MIN..MAX moments only. part: [share][row][column], times scale.
 // Bound by the FP64 pipe: 2 J + about 2 multiply-adds a pixel and visibility,
 // where reduction and sincospi took about 59. 500 x 500 pixels, 20,000
 // visibilities: 15.9 -> 3.5 ms.
@@ -240,8 +249,9 @@ template <int MIN, int MAX>
 __global__ void __launch_bounds__(128) dft_moments_kernel(const double *__restrict__ u, const double *__restrict__ v,
                                                           const double *__restrict__ w,
                                                           const double2 *__restrict__ vis, int64_t nvis,
-                                                          double *__restrict__ part, int N, double theta, int row0,
-                                                          int nrows, const double *__restrict__ wmax_p)
+                                                          double *__restrict__ part, int N, double theta,
+                                                          double scale, int row0, int nrows,
+                                                          const double *__restrict__ wmax_p)
 {
     __shared__ double2 sC[kDftVis][TILE];
     __shared__ double sB[2 * kDftVis][kDftStrideB];
@@ -338,17 +348,16 @@ __global__ void __launch_bounds__(128) dft_moments_kernel(const double *__restri
                 // Re((-i)^j (re + i im)): re, im, -re, -im
                 sum = fma(j & 2 ? -f : f, mom, sum);
             }
-            part[((int64_t)blockIdx.z * nrows + (y - row0)) * N + x] = sum;
+            part[((int64_t)blockIdx.z * nrows + (y - row0)) * N + x] = scale * sum;
         }
 }
 
-// image = factor * the sum of the shares, in order, for the tiles of the moments
-// (part may be image, of one share)
-__global__ void dft_shares_kernel(const double *part, int shares, double *image, int N,
-                                  double theta, double factor, int row0, int nrows, const double *__restrict__ wmax)
+// image = factor * the sum of the shares, in order
+__global__ void dft_shares_kernel(const double *__restrict__ part, int shares, double *__restrict__ image, int N,
+                                  double factor, int nrows)
 {
-    const int x = blockIdx.x * TILE + threadIdx.x % TILE, tile_y = row0 + blockIdx.y * TILE;
-    if (dft_moments(blockIdx.x * TILE, tile_y, N, theta, *wmax) == 0 || x >= N) return;
+    const int x = blockIdx.x * TILE + threadIdx.x % TILE;
+    if (x >= N) return;
     for (int y = blockIdx.y * TILE + threadIdx.x / TILE; y < min(nrows, (int)(blockIdx.y + 1) * TILE); y += 8) {
         double s = 0.0;
         for (int k = 0; k < shares; k++) s += part[((int64_t)k * nrows + y) * N + x];
@@ -356,16 +365,39 @@ __global__ void dft_shares_kernel(const double *part, int shares, double *image,
     }
 }
 
+// Tiles of the whole image: the rules below go by it, so a band of rows is summed
+// as the image's rows are.
+static int64_t dft64_tiles(int grid_size)
+{
+    const int64_t side = (grid_size + TILE - 1) / TILE;
+    return side * side;
+}
+
 // Shares the visibilities are split into: six rounds of four resident CTAs an SM
-// over the whole image's tiles, for a short tail (three rounds: 3.64 against 3.48
-// ms at 500 x 500), at least 512 visibilities each. The whole image's, so
-// a band of rows is summed as the image's rows are.
+// over the tiles, for a short tail (three rounds: 3.64 against 3.48 ms at
+// 500 x 500), at least 512 visibilities each. Below 1024 visibilities that is one
+// share, whose tiles go through them one after another: one round there, at
+// least 32 each. 64 x 64, 400 visibilities: 143 -> 68 us; 380 x 380, 400: 104 ->
+// 90; the same on larger calls would cost (100 x 100, 5000: 184 -> 229 us).
 int dft64_shares(int grid_size, int64_t n, int sm_count)
 {
-    const int64_t tiles = (int64_t)((grid_size + TILE - 1) / TILE) * ((grid_size + TILE - 1) / TILE);
+    const int64_t tiles = dft64_tiles(grid_size);
     int64_t s = ((int64_t)sm_count * 24 + tiles - 1) / tiles;
     if (s > n / 512) s = n / 512;
+    if (n < 1024) s = std::min<int64_t>((int64_t)sm_count * 4 / tiles, n / 32);
     return s < 1 ? 1 : (int)(s > 64 ? 64 : s);
+}
+
+// FP64, pixel by pixel for the whole image, where the visibilities are too few to
+// pay for the moments' launches, 20 us: a tile takes 0.47 us a visibility so,
+// about half of that by moments (8 x 8 pixels, 1 visibility: 24 against 43 us;
+// 16 x 16, 64: 53 against 73; 200 x 200, 64 and 96: 53 and 65 against 53 and 49;
+// 500 x 500, 10: 29 against 41). Up to 16 tiles, at most 128 pixels a side, the
+// line lies higher, such tiles needing more moments (128 x 128, 96: 68 against 74).
+static bool dft64_by_pixel(int grid_size, int64_t n, int sm_count)
+{
+    const int64_t tiles = dft64_tiles(grid_size);
+    return tiles <= 16 ? n <= 96 : n * std::max<int64_t>(tiles, sm_count) <= (int64_t)64 * sm_count;
 }
 
 void launch_dft(cudaStream_t s, const double *u, const double *v, const double *w,
@@ -384,19 +416,26 @@ void launch_dft(cudaStream_t s, const double *u, const double *v, const double *
                                                                  nrows, nullptr);
             break;
         case RG_DFT_FP64: {
+            if (dft64_by_pixel(grid_size, n, sm_count)) {
+                dft_kernel<RG_DFT_FP64><<<grd, 256, 0, s>>>(u, v, w, vis, n, image, grid_size, theta, factor, row0,
+                                                            nrows, nullptr);
+                break;
+            }
             const int shares = dft64_shares(grid_size, n, sm_count);
-            double *wmax = work, *part = shares > 1 ? work + 2 : image;  // one share: summed in place
+            double *wmax = work, *part = shares > 1 ? work + 2 : image;
+            const double scale = shares > 1 ? 1.0 : factor;  // one share: the image itself
             cudaMemsetAsync(wmax, 0, sizeof(double), s);
             if (n > 0)
                 dft_range_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 592), 256, 0, s>>>(
                     u, v, w, vis, n, (unsigned long long *)wmax);
             const dim3 tiles(grd.x, grd.y, shares);
-            dft_moments_kernel<1, 4><<<tiles, 128, 0, s>>>(u, v, w, vis, n, part, grid_size, theta, row0, nrows, wmax);
-            dft_moments_kernel<5, kDftMoments><<<tiles, 128, 0, s>>>(u, v, w, vis, n, part, grid_size, theta, row0,
-                                                                    nrows, wmax);
-            dft_shares_kernel<<<grd, 256, 0, s>>>(part, shares, image, grid_size, theta, factor, row0, nrows, wmax);
-            dft_kernel<RG_DFT_FP64><<<grd, 256, 0, s>>>(u, v, w, vis, n, image, grid_size, theta, factor, row0, nrows,
-                                                        wmax);
+            dft_moments_kernel<1, 4><<<tiles, 128, 0, s>>>(u, v, w, vis, n, part, grid_size, theta, scale, row0, nrows,
+                                                           wmax);
+            dft_moments_kernel<5, kDftMoments><<<tiles, 128, 0, s>>>(u, v, w, vis, n, part, grid_size, theta, scale,
+                                                                    row0, nrows, wmax);
+            dft_kernel<RG_DFT_FP64><<<tiles, 256, 0, s>>>(u, v, w, vis, n, part, grid_size, theta, scale, row0, nrows,
+                                                          wmax);
+            if (shares > 1) dft_shares_kernel<<<grd, 256, 0, s>>>(part, shares, image, grid_size, factor, nrows);
             break;
         }
         default:

@@ -154,6 +154,28 @@ def test_dft_fp64_tiles_vs_numpy(rg, ctx, n, nv, th, wmax):
         assert np.array_equal(ctx.dft_image_rows(n, th, V, 32, n - 32, rg.RG_DFT_FP64), img[32:], equal_nan=True)
 
 
+# some tiles by moments and some pixel by pixel, in one share of the visibilities
+# and in several; few visibilities, up to the line below which every tile goes
+# pixel by pixel, on an image of a tile and of more tiles than SMs. Tolerance as
+# above.
+@pytest.mark.parametrize("n,nv,th,wmax", [(128, 400, 0.5, 100.0), (130, 2100, 0.5, 100.0), (160, 1600, 1.5, 1.0),
+                                          (32, 96, 0.1, 100.0), (32, 97, 0.1, 100.0), (129, 64, 0.1, 100.0),
+                                          (129, 65, 0.1, 100.0), (390, 55, 0.1, 100.0), (390, 60, 0.1, 100.0), (70, 1023, 0.1, 50.0),
+                                          (70, 1024, 0.1, 50.0)])
+def test_dft_fp64_mixed_tiles_vs_numpy(rg, ctx, n, nv, th, wmax):
+    rng = np.random.default_rng(7 * n + nv)
+    u, v = rng.uniform(-0.5 * n / th, 0.5 * n / th, (2, nv))
+    w = rng.uniform(-wmax, wmax, nv)
+    vis = rng.normal(size=nv) + 1j * rng.normal(size=nv)
+    V = rg.Visibilities(u, v, w, vis)
+    img = ctx.dft_image(n, th, V, rg.RG_DFT_FP64, 2.0)
+    ref = _dft64_numpy(n, th, u, v, w, vis)
+    assert np.array_equal(np.isnan(img), np.isnan(ref))
+    assert np.nanmax(np.abs(img - ref)) < 1e-12 * np.nanmax(np.abs(ref))
+    if n > 32:
+        assert np.array_equal(ctx.dft_image_rows(n, th, V, 32, n - 32, rg.RG_DFT_FP64), img[32:], equal_nan=True)
+
+
 def test_dft_fp64_non_finite_and_empty_inputs(rg, ctx):
     n, th = 40, 0.1
     u, v, w = np.array([10.0, 20.0]), np.array([-5.0, 3.0]), np.array([1.0, 2.0])
