@@ -2,10 +2,13 @@
 restatement of the reference's wstack_predict (src/wstack/predict.cpp:
 396-562) with the same kernels: FP64 on both sides, so the visibilities
 agree to rounding; and against the direct sum over the quantised sky."""
+import functools
+import types
+
 import numpy as np
 import pytest
 
-from test_wstack_oracle import case
+from test_wstack_oracle import case, numpy_predict
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +82,32 @@ def test_refused_visibility_is_zero_beside_an_infinite_source(rg, ctx, sim, nv, 
     zero = np.zeros(nv, bool)
     zero[[nv // 2, nv - 1]] = True
     assert np.all(out[zero] == 0) and not np.isfinite(out[~zero]).any()
+
+
+@pytest.fixture(scope="module")
+def tables(sim):
+    """The separable kernels, each made once (seconds)."""
+    return types.SimpleNamespace(sepkern_pswf=functools.lru_cache(None)(sim.sepkern_pswf))
+
+
+# Each way by name, far from where the rule changes over (a factor of three or
+# more in the times it compares). Direct: every class of supports, 32 sources
+# several times over with a remainder. Stack: many sources, or supports beyond the
+# direct kernel's 16; powers of two, and lengths for Bluestein's algorithm, up to
+# the largest stack.
+@pytest.mark.parametrize("way,lam,nv,npts,suv,sw,dw", [
+    ("direct", 5120.0, 300, 70, 12, 4, 50.0), ("direct", 5120.0, 100, 130, 8, 6, 50.0),
+    ("direct", 5120.0, 257, 64, 8, 8, 50.0), ("direct", 5120.0, 100, 33, 12, 12, 50.0),
+    ("stack", 5120.0, 200, 3000, 8, 6, 50.0), ("stack", 10240.0, 100, 40, 18, 4, 30.0),
+    ("stack", 10300.0, 100, 40, 18, 4, 30.0), ("stack", 20480.0, 50, 20, 18, 4, 60.0),
+    ("stack", 20420.0, 50, 20, 18, 4, 60.0)])
+def test_predict_ways_match_numpy(rg, tables, way, lam, nv, npts, suv, sw, dw):
+    c = case(tables, seed=nv + npts, lam=lam, nv=nv, npts=npts, suv=suv, sw=sw, dw=dw)
+    ctx = rg.Context(0)  # its own: the largest stack's memory goes with it
+    ctx.set_profiling(True)
+    got = _run(ctx, c)
+    stages = [s for s, _ in ctx.last_timings()]
+    ctx.close()
+    assert stages == (["wstack_direct"] if way == "direct" else ["wstack_fft", "wstack_degrid"])
+    ref = numpy_predict(c)
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-11
