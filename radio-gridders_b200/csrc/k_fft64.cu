@@ -121,6 +121,11 @@ struct StCols {
     __device__ void operator()(int arr, int line, int n, double2 v) const { d[arr * array + n * ld + line] = v; }
 };
 
+void launch_fft64_rows(cudaStream_t s, double2 *data, const Fft64Plan &p, int rows, int sign)
+{
+    launch_fft64_lines<false>(s, p, 1, rows, sign, LdRows{data, p.n}, StRows{data, p.n});
+}
+
 rg_status roots64(rg_context *ctx, int n, const double2 **out)
 {
     const std::string name = "roots64_" + std::to_string(n);
@@ -186,7 +191,7 @@ rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out)
         fft64_chirp_kernel<<<(p.L + 127) / 128, 128, 0, ctx->stream>>>(chirp, filter, n, p.L);
         Fft64Plan q = p;  // the L-point transform of the filter
         q.n = p.L;
-        launch_fft64_lines<false>(ctx->stream, q, 1, 1, -1, LdRows{filter, p.L}, StRows{filter, p.L});
+        launch_fft64_rows(ctx->stream, filter, q, 1, -1);
         p.filter = filter;
         p.chirp = chirp;
     }
@@ -207,7 +212,7 @@ void launch_fft64_2d(cudaStream_t s, double2 *data, int batch, const Fft64Plan &
     for (int64_t at = 0; at < batch; at += step) {
         const int cnt = (int)std::min<int64_t>(step, batch - at);
         double2 *d = data + at * array;
-        launch_fft64_lines<false>(s, px, 1, cnt * ny, sign, LdRows{d, nx}, StRows{d, nx});
+        launch_fft64_rows(s, d, px, cnt * ny, sign);
         launch_fft64_lines<true>(s, py, cnt, nx, sign, LdCols{d, nx, array}, StCols{d, nx, array});
     }
 }

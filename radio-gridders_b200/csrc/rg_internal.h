@@ -236,6 +236,8 @@ bool fft64_smooth(int n);  // no prime factor above 7: transformed directly
 rg_status roots64(rg_context *ctx, int n, const double2 **out);
 // The context's plan for length n (its tables are made on the first call).
 rg_status fft64_plan(rg_context *ctx, int n, Fft64Plan *out);
+// In-place transforms of consecutive rows of p.n points (at most 2^30 rows).
+void launch_fft64_rows(cudaStream_t s, double2 *data, const Fft64Plan &p, int rows, int sign);
 // In-place 2-D transforms of `batch` ny x nx arrays.
 void launch_fft64_2d(cudaStream_t s, double2 *data, int batch, const Fft64Plan &py, const Fft64Plan &px, int sign);
 // The dirty image of an n x n grid (n even): hermitian sum, shift, transform

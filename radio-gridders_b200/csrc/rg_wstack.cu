@@ -93,16 +93,6 @@ struct StStackCol {
         stack[((int64_t)arr * G + y) * G + x] = v;
     }
 };
-struct LdSkyRow {
-    const double2 *d;
-    int64_t ld;
-    __device__ double2 operator()(int, int line, int n) const { return d[line * ld + n]; }
-};
-struct StSkyRow {
-    double2 *d;
-    int64_t ld;
-    __device__ void operator()(int, int line, int n, double2 v) const { d[line * ld + n] = v; }
-};
 
 // The geometry and kernel tables of the de-convolution.
 struct DegridGeom {
@@ -494,8 +484,7 @@ extern "C" rg_status rg_wstack_predict(rg_context *ctx, double theta, double lam
             const int64_t tot = (int64_t)nsrc * planes;
             wstack_scatter_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 4096), 256, 0, st>>>(
                 (const SkyEntry *)d_sky, nsrc, planes, t0, N, G, nrows, theta, dw, (double2 *)rows);
-            launch_fft64_lines<false>(st, plan, 1, planes * nrows, -1, LdSkyRow{(const double2 *)rows, G},
-                                      StSkyRow{(double2 *)rows, G});
+            launch_fft64_rows(st, (double2 *)rows, plan, planes * nrows, -1);
             ctx->launches += 2;
         }
         launch_fft64_lines<true>(st, plan, planes, G, -1,
