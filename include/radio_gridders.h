@@ -428,11 +428,13 @@ typedef struct rg_sepkern {
  * round(0.5 / x0) times floor(theta lambda) pixels, one FP64 FFT per w plane
  * (planes every dw; ceil(sin(theta/2) sqrt(2) N / dw) + conv_w.size + 1 of
  * them), then per visibility the separable conv_w x conv_uv^2 sum over the
- * stack (du: the uv cell of the padded grid).  Replaces wstack_predict
+ * stack (du: the uv cell of the padded grid); few sources are summed at each
+ * visibility's taps without a stack, to the same values within FP64 rounding.  Replaces wstack_predict
  * (src/wstack/predict.cpp:396-562) and wstack_predict_cu_3D
  * (src/wstack/predict.cu:808-1081).  vis_out: 2*nvis doubles.  FP64.
  * RG_ERR_INVALID_ARGUMENT for a source outside the image or a visibility
- * whose taps leave the stack (the reference reads past its arrays). */
+ * whose taps leave the stack (the reference reads past its arrays; such a
+ * visibility is zero in vis_out). */
 rg_status rg_wstack_predict(rg_context *ctx, double theta, double lambda, const double *points, int npoints,
                             const double *u, const double *v, const double *w, int64_t nvis, double du, double dw,
                             double x0, const rg_sepkern *conv_uv, const rg_sepkern *conv_w,

@@ -21,7 +21,7 @@
 //     accumulated in FP64.
 //   FP32_NAIVE: phi formed in FP32 from FP32 u, v, w, l, m, n, reduced in FP32.
 //   FP64: phi, reduction and sin/cos all FP64, per pixel and visibility only
-//     where the tiles below do not apply.
+//     where the tiles below do not apply or the visibilities are few.
 //
 // FP64 by tiles. Over a 32 x 32 tile the phase is separable but for a small
 // rest: with g(l, m) = 1 - n and the tile's centre (l0, m0),
@@ -242,7 +242,8 @@ __device__ __forceinline__ double turns(double a, double b, double c)
 // MIN..MAX moments only. part: [share][row][column], times scale.
 // Bound by the FP64 pipe: 2 J + about 2 multiply-adds a pixel and visibility,
 // where reduction and sincospi took about 59. 500 x 500 pixels, 20,000
-// visibilities: 15.9 -> 3.5 ms.
+// visibilities: 15.9 -> 3.5 ms, the products at 0.66 of the pipe's rate and the
+// phasors 0.16 of its cycles.
 constexpr int kDftVis = 32, kDftStrideB = TILE + 4;  // 4 mod 16: a fragment's 4 k x 8 rows on distinct banks
 
 template <int MIN, int MAX>

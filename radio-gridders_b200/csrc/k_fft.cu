@@ -344,8 +344,8 @@ __global__ void __launch_bounds__(kSparseColThreads) sparse_cols_kernel(
 // visibilities: 92 -> 28 us (there one warp of four had done all of step 1).
 //
 // tower_rows_finish_kernel: CTA = (tower, strip of R rows).  Sums the tower's
-// group partials in group order (deterministic) and applies the forward row transform into the tower's sub-image (the
-// row half of grid.c:499).
+// group partials in group order (deterministic) and applies the forward row
+// transform into the tower's sub-image (the row half of grid.c:499).
 // ---------------------------------------------------------------------------
 constexpr int kRowThreads = 128;
 template <int N1>
@@ -361,7 +361,7 @@ struct RowGeom {
     static constexpr int T_ELEMS = kRowThreads * kPad;
 };
 
-int tower_row_strips(int subgrid) { return subgrid / (subgrid >= 1024 ? 4 : 8); }
+int tower_group_strips(int subgrid) { return subgrid / (subgrid >= 1024 ? 4 : 8); }
 
 // Bit n2 (n2 < 32) of the result = strip (n1 + n2*N1)/kStripCols of the
 // 128-bit strip mask (lo, hi) is marked: the element n1 + n2*N1 of a row that

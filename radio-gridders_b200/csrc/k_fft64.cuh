@@ -359,7 +359,7 @@ int fft64_threads(const Fft64Plan &p, int lgT)
 
 // Lines a CTA takes: up to 8192 points (2048 for rows, whose lines need no
 // neighbour) and 8 columns (128-byte pieces of a row), fewer while the launch
-// would leave SMs without a CTA. Two columns at least where they fit, so a
+// would leave an SM (of 148) without two CTAs. Two columns at least where they fit, so a
 // 32-byte sector is read once.
 inline int fft64_lines_lg(const Fft64Plan &p, bool col, int64_t lines)
 {

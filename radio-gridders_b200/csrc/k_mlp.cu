@@ -66,7 +66,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Four (two) 8 x 8 tiles of 16-bit elements from shared memory, each lane giving
+// Four 8 x 8 tiles of 16-bit elements from shared memory, each lane giving
 // the address of one row of one tile; T: transposed.
 template <bool T>
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const bf16 *row)
@@ -233,7 +233,7 @@ __device__ __forceinline__ void tap_features_tab(float w, float du, float dv, in
     for (int k = MNFEAT; k < MFIN; k++) f[k] = to_elem<T>(0.f);
 }
 
-// Epilogue of a 32x32 (per warp) hidden-layer tile: z = acc + b; Z (fp32,
+// Epilogue of a warp's WM x WN hidden-layer tile: z = acc + b; Z (fp32,
 // optional) and H = bf16(silu(z)).
 template <int WM, int WN>
 __device__ __forceinline__ void hidden_epilogue(const float (&acc)[WM / 16][WN / 8][4], int m0, int n0,

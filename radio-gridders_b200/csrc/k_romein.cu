@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(K *K / P, (RomeinBounds<K, P>::min_ctas)) rome
 }
 
 // Row-major grids, supports of 16 and 32, with a converted table in the paired
-// layout (launch_convert_table_pairs): entry [r][c], r < K/2, of a slice holds the
+// layout (launch_convert_taps): entry [r][c], r < K/2, of a slice holds the
 // taps of rows r and r + K/2 as (re, re, im, im). A thread's points are taken in
 // pairs K/2 rows apart, so one 16-byte load brings both taps ready for packed
 // multiply-adds whose other operands, (re, re), (im, im) and (-re, -re) of the

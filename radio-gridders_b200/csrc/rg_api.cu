@@ -561,7 +561,7 @@ static rg_status wtowers_enqueue(rg_context *ctx, const DevVis &dv, const float2
     end_stage(ctx);
     begin_stage(ctx, "compact");
     launch_compact_bins(st, (const int *)active, range, (int *)slot_of_bin, (int *)bin_of_slot, counts,
-                        (int *)tfirst, (int *)tcount, ntowers, tower_row_strips(S), pl.tune.group_items * ctx->sm_count,
+                        (int *)tfirst, (int *)tcount, ntowers, tower_group_strips(S), pl.tune.group_items * ctx->sm_count,
                         (int *)gbegin,
                         (int *)gend, (int *)tgfirst, (int *)tgcount);
     end_stage(ctx);

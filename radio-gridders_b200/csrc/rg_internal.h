@@ -71,7 +71,7 @@ rg_status grid_wtowers_impl(rg_context *ctx, double *uvgrid, int grid_size, doub
 // Schedule knobs of a W-towers pass (picked by the autotuner).
 struct TowerTuning {
     int romein_points = 8;  // grid points per Romein thread (threads per CTA = K^2 / points)
-    int group_items = 8;    // row-stage work items per SM (sets the floor-group size)
+    int group_items = 8;    // work items per SM (tower_group_strips; sets the floor-group size)
 };
 
 struct TowerPlan {
@@ -340,7 +340,11 @@ void launch_tower_rows(cudaStream_t s, float2 *slots, const unsigned *masks, con
 void launch_tower_finish(cudaStream_t s, int group_cap, const int *tower_group_first,
                          const int *tower_group_count, int ntowers, const float2 *partial,
                          float2 *subimg, int subgrid, const float2 *tw);
-int tower_row_strips(int subgrid);  // row strips per sub-grid in the row stage
+// Strips of the group sums (FinishGeom): what the floor groups are sized by. The
+// row stage takes S^2 / 4096 strips a sub-grid, fewer below S = 512, so a work item
+// of the schedule counts 2 to 8 of its CTAs there; the measure stays, and with it
+// the groups and the order in which floors are summed. The tuner picks the items by time.
+int tower_group_strips(int subgrid);
 void launch_add_back(cudaStream_t s, const float2 *subimg, const int *tower_count,
                      double2 *master, int grid_size, int subgrid, int margin, int chunk,
                      int nchunk, int overwrite, const int *range, const int *counts, int slot_cap,

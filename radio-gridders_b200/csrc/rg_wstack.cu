@@ -205,8 +205,9 @@ __device__ __forceinline__ double2 zmul(double2 a, double2 b)
 // Bound by the FP64 pipe (2 (2 SU + SW) + 18 multiply-adds a source and
 // visibility) and, close behind, by shared memory, whose broadcast reads two
 // visibilities a thread share. 50 sources and 200,000 visibilities
-// (supports 8, 8, 6; G = 2048, 15 planes): 88 us with its set-up, 78 % of the
-// FP64 pipe's rate in the long run; the whole call 5450 -> 138 us.
+// (supports 8, 8, 6; G = 2048, 15 planes): 88 us with its set-up, the FP64
+// pipe busy for half of its cycles (782 CTAs in two rounds of 444; 400 sources
+// run at 0.53 of its rate); the whole call 5450 -> 138 us.
 constexpr int kDirectThreads = 128, kDirectSources = 32;
 
 template <int SU, int SW, int V>
