@@ -108,8 +108,9 @@ def fake(tmp_path_factory):
     d = tmp_path_factory.mktemp("fake")
     (d / "fake.cpp").write_text(FAKE)
     so = str(d / "fake.so")
-    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I/usr/local/cuda/include", "-I", os.path.join(PKG, "csrc"),
-                    "-o", so, str(d / "fake.cpp"), obj], check=True)
+    # bound within the file: another library of the process may hold the real runtime
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I/usr/local/cuda/include", "-I",
+                    os.path.join(PKG, "csrc"), "-o", so, str(d / "fake.cpp"), obj], check=True)
     return ct.CDLL(so)
 
 
